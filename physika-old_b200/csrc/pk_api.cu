@@ -293,7 +293,7 @@ PK_API int pk_ctx_destroy(pk_ctx* c)
                     c->rows, c->hits, c->hpool, c->rpool, c->ovf, c->ovf_list, c->spill, c->tile_cnt,
                     c->tile_off, c->tiles, c->cell_cnt, c->cell_start, c->scan_part, c->g_rho, c->g_lam,
                     c->g_dpos, c->g_xold, c->sdf, c->pd_index, c->pd_rest_idx, c->pd_rest_pos,
-                    c->pd_alive, c->pd_invK, c->pd_bulk, c->pd_xold, c->pd_delta, c->pd_w,
+                    c->pd_alive, c->pd_invK, c->pd_bulk, c->pd_bond, c->pd_raw,
                     c->pd_in_cnt, c->pd_in_off, c->pd_in, c->pd_in_slot, c->h_x, c->h_v, c->pd_ktw, c->pl_mk};
     pk::pd_work_release(c);
     pk::pbd_roll_release(c);
@@ -1090,7 +1090,7 @@ PK_API int pk_pd_init(pk_ctx* c, const float* x, int n, const int* index, const 
     if (n > c->pd_cap_n) {
         size_t m = (size_t)n;
         if (!(regrow(c->pd_index, m) && regrow(c->pd_invK, 9 * m) && regrow(c->pd_bulk, m) &&
-              regrow(c->pd_xold, 3 * m) && regrow(c->pd_delta, 3 * m) && regrow(c->pd_w, m) && regrow(c->pd_ktw, m) &&
+              regrow(c->pd_ktw, m) &&
               regrow(c->pd_in_cnt, m + 1) && regrow(c->pd_in_off, m + 1))) {
             c->pd_cap_n = 0;
             return fail(c, PK_ERR_NOMEM, "device allocation of elasticity state failed");
@@ -1105,7 +1105,7 @@ PK_API int pk_pd_init(pk_ctx* c, const float* x, int n, const int* index, const 
         c->pd_cap_rest = bonds;
     }
     if (bonds > c->pd_cap_bonds) {
-        if (!(regrow(c->pd_alive, (size_t)bonds) && regrow(c->pd_in, (size_t)bonds) &&
+        if (!(regrow(c->pd_alive, (size_t)bonds) && regrow(c->pd_raw, (size_t)bonds) && regrow(c->pd_in, (size_t)bonds) &&
               regrow(c->pd_in_slot, (size_t)bonds))) {
             c->pd_cap_bonds = 0;
             return fail(c, PK_ERR_NOMEM, "device allocation of the bond masks failed");
@@ -1113,6 +1113,7 @@ PK_API int pk_pd_init(pk_ctx* c, const float* x, int n, const int* index, const 
         c->pd_cap_bonds = bonds;
     }
     c->pd_n = n;
+    ++c->pd_shape_rev;
     c->pd_begun = false;
     if (c->pl_yield && n > 0 && n <= c->pl_cap_n)  // m_bYield.reset() (ElastoplasticityModule.cu:665)
         cudaMemsetAsync(c->pl_yield, 0, (size_t)n, (cudaStream_t)stream);
@@ -1200,6 +1201,7 @@ PK_API int pk_pd_rollout_backward(pk_ctx* c, const float* xbar, const float* vba
         return fail(c, PK_ERR_ARG, "null adjoint or gradient arrays");
     cudaSetDevice(c->device);
     c->launches = pk::pd_backward_f32(c, xbar, vbar, grad_x0, grad_v0, grad_bulk, (cudaStream_t)stream);
+    if (c->launches == -2) return fail(c, PK_ERR_NOMEM, "device allocation of the reverse pass failed");
     if (c->launches < 0) return fail(c, PK_ERR_STATE, "no checkpointed float rollout to differentiate");
     return check_launch(c, "pk_pd_rollout_backward");
 }
@@ -1228,6 +1230,7 @@ PK_API int pk_pd_rollout_backward_f64(pk_ctx* c, const double* xbar, const doubl
         return fail(c, PK_ERR_ARG, "null adjoint or gradient arrays");
     cudaSetDevice(c->device);
     c->launches = pk::pd_backward_f64(c, xbar, vbar, grad_x0, grad_v0, grad_bulk, (cudaStream_t)stream);
+    if (c->launches == -2) return fail(c, PK_ERR_NOMEM, "device allocation of the reverse pass failed");
     if (c->launches < 0) return fail(c, PK_ERR_STATE, "no checkpointed double rollout to differentiate");
     return check_launch(c, "pk_pd_rollout_backward_f64");
 }
@@ -1342,6 +1345,7 @@ PK_API int pk_pd_rotate_rest_shape(pk_ctx* c, const float* x, int n, float horiz
     if (n > 0 && !x) return fail(c, PK_ERR_ARG, "null positions");
     cudaSetDevice(c->device);
     if ((rc = ensure_plastic(c))) return rc;
+    ++c->pd_shape_rev;
     c->launches = pk::pl_rotate(c, x, horizon, (cudaStream_t)stream);
     return check_launch(c, "pk_pd_rotate_rest_shape");
 }
@@ -1353,6 +1357,7 @@ PK_API int pk_pd_apply_yielding(pk_ctx* c, const float* x, int n, const pk_plast
     if (rc) return rc;
     cudaSetDevice(c->device);
     if ((rc = ensure_plastic(c))) return rc;
+    ++c->pd_shape_rev;
     c->launches = pk::pl_yield(c, x, p, (cudaStream_t)stream);
     return check_launch(c, "pk_pd_apply_yielding");
 }
@@ -1407,11 +1412,13 @@ PK_API int pk_pd_reconstruct_rest_shape(pk_ctx* c, const float* x, int n, const 
     }
     l += pk::pl_recon_fill(c, x, index, elements, cap, total, st);
     // the new shape becomes the rest shape (CSR); the old buffers are the next spares
+    ++c->pd_shape_rev;
     std::swap(c->pd_rest_idx, c->pl_rest_idx2);
     std::swap(c->pd_rest_pos, c->pl_rest_pos2);
     std::swap(c->pd_cap_rest, c->pl_cap_rest2);
     if (new_total > c->pd_cap_bonds) {
-        if (!(regrow(c->pd_alive, (size_t)new_total) && regrow(c->pd_in, (size_t)new_total) &&
+        if (!(regrow(c->pd_alive, (size_t)new_total) && regrow(c->pd_raw, (size_t)new_total) &&
+              regrow(c->pd_in, (size_t)new_total) &&
               regrow(c->pd_in_slot, (size_t)new_total))) {
             c->pd_cap_bonds = 0;
             return fail(c, PK_ERR_NOMEM, "device allocation of the bond masks failed");

@@ -113,9 +113,13 @@ struct pk_ctx {
     unsigned char* pd_alive = nullptr;
     float* pd_invK = nullptr;      // 9 per particle, row-major
     float* pd_bulk = nullptr;
-    float* pd_xold = nullptr;
-    float* pd_delta = nullptr;
-    float* pd_w = nullptr;
+    // The projection's compact bonds (pk_pd_adj.cu: rest vector and neighbour),
+    // derived from the rest shape: pd_shape_rev counts the shape's changes,
+    // pd_bond_rev says which of them the bonds hold.
+    float4* pd_bond = nullptr;
+    long long pd_bond_cap = 0;
+    int* pd_raw = nullptr;         // place in the rest shape of every compact bond
+    unsigned long long pd_shape_rev = 1, pd_bond_rev = 0;
     float* pd_ktw = nullptr;  // computeInverseK: the weight sum between its two kernels
     float pd_horizon = 0.0f;
     long long pd_cap_bonds = 0;    // capacity of pd_alive and pd_in

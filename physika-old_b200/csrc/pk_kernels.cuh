@@ -75,7 +75,7 @@ int pl_recon_fill(pk_ctx* c, const float* x, const int* nindex, const int* nelem
                   cudaStream_t st);
 int pl_fill_alive(pk_ctx* c, long long bonds, cudaStream_t st);
 int pd_project_solve(pk_ctx* c, float* x, float* v, int n, float horizon, float mu, float lambda, int iterations,
-                     float dt, cudaStream_t st);
+                     float dt, float stretch, cudaStream_t st);
 int pd_rollout_f32(pk_ctx* c, float* x, float* v, int n, const float g[3], const pk_pd_params* p, int steps,
                    int every, cudaStream_t st);
 int pd_rollout_f64(pk_ctx* c, double* x, double* v, const double* bulk, int n, const double g[3],

@@ -129,34 +129,6 @@ __global__ void __launch_bounds__(256) k_fill_u8(unsigned char* __restrict__ p, 
     if (t < m) p[t] = v;
 }
 
-// Stretch break (no reference counterpart): a bond dies for good once
-// |x_i - x_j| > (1 + s) * |rest_i - rest_j|.  kBreakG lanes per particle,
-// lane `sub` taking bonds sub, sub + kBreakG, ...
-constexpr int kBreakG = 8;
-__global__ void __launch_bounds__(256)
-    k_pd_break(const float* __restrict__ x, int n, const int* __restrict__ index, int cap,
-               long long total, const int* __restrict__ ridx, const float* __restrict__ rpos,
-               unsigned char* __restrict__ alive, float s)
-{
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = (int)(gid / kBreakG), sub = (int)(gid % kBreakG);
-    if (i >= n) return;
-    long long a0 = pd_at(index, cap, i, 0);
-    int m = pd_size(index, cap, total, n, i);
-    for (int e = sub; e < m; e += kBreakG) {
-        long long at = pd_at(index, cap, i, e);
-        if (!alive[at]) continue;
-        int j = ridx[at];
-        float r0 = rpos[3 * at] - rpos[3 * a0], r1 = rpos[3 * at + 1] - rpos[3 * a0 + 1],
-              r2 = rpos[3 * at + 2] - rpos[3 * a0 + 2];
-        float c0 = x[3 * j] - x[3 * i], c1 = x[3 * j + 1] - x[3 * i + 1], c2 = x[3 * j + 2] - x[3 * i + 2];
-        // lengths rounded as Vector3f::norm compiles (fma(z,z,fma(x,x,y*y)))
-        float lr = __fsqrt_rn(__fmaf_rn(r2, r2, __fmaf_rn(r0, r0, __fmul_rn(r1, r1))));
-        float lc = __fsqrt_rn(__fmaf_rn(c2, c2, __fmaf_rn(c0, c0, __fmul_rn(c1, c1))));
-        if (lc > __fmul_rn(__fadd_rn(1.0f, s), lr)) alive[at] = 0;
-    }
-}
-
 int pd_rest_shape(pk_ctx* c, const float* x, int n, const int* index, const int* elements, int cap,
                   long long total, float horizon, cudaStream_t st)
 {
@@ -183,17 +155,8 @@ int pd_solve(pk_ctx* c, float* x, float* v, int n, float horizon, float mu, floa
              int iterations, float dt, float break_stretch, cudaStream_t st)
 {
     if (n <= 0) return 0;
-    int launches = 0;
-    if (break_stretch > 0.f) {
-        k_pd_break<<<(unsigned)(((long long)n * kBreakG + 255) / 256), 256, 0, st>>>(x, n, c->pd_index, c->pd_cap,
-                                                                                      c->pd_total,
-                                                               c->pd_rest_idx, c->pd_rest_pos, c->pd_alive,
-                                                               break_stretch);
-        ++launches;
-    }
     // the projection as gathers over outgoing and incoming bonds (pk_pd_adj.cu)
-    const int l = pd_project_solve(c, x, v, n, horizon, mu, lambda, iterations, dt, st);
-    return l < 0 ? l : launches + l;
+    return pd_project_solve(c, x, v, n, horizon, mu, lambda, iterations, dt, break_stretch, st);
 }
 
 }  // namespace pk

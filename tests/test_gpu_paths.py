@@ -1,0 +1,84 @@
+"""The branches that sizes and histories take: bond rows too long to be ordered,
+and broken bonds seen by the step-by-step projection.  The oracle is the CPU
+restatement; where two paths of the library must agree, they agree bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+import pkhot
+import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def t(a, dtype=np.float32):
+    return torch.from_numpy(np.ascontiguousarray(a, dtype)).cuda()
+
+
+def rel(a, b):
+    return float(np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-30))
+
+
+def bar(ctx, oracle, ratio, cap, seed=0):
+    sc = scenes.elastic_bar(seed=seed, dims=(9, 8, 7), cap=cap)
+    h = ratio * sc.spacing
+    x = (sc.x + np.random.default_rng(seed).uniform(-0.02, 0.02, sc.x.shape) * sc.spacing).astype(np.float32)
+    ri, re = oracle.neighbor_query(x, h, sc.lo, sc.hi, cap)
+    ctx.pd_init(t(x), t(ri, np.int32), t(re, np.int32), cap, re.shape[0], h)
+    ctx.pd_set_bulk(t(sc.bulk))
+    return sc, x, h, ri, re
+
+
+@pytest.mark.parametrize("ratio,cap", [(1.2, 0), (3.0, 7), (3.0, 80), (4.6, 0)])
+def test_projection_of_short_and_long_bond_rows(ctx, oracle, ratio, cap):
+    # 7 bonds to about 250: less than a batch, one odd batch, rows past 128
+    sc, x0, h, ri, re = bar(ctx, oracle, ratio, cap, seed=4)
+    v0 = np.random.default_rng(4).normal(0, 0.05, x0.shape).astype(np.float32)
+    oidx, opos = oracle.pd_rest_shape(x0, ri, re, cap)
+    oinv = oracle.pd_inverse_k(ri, cap, re.shape[0], opos, h)
+    x, v = t(x0), t(v0)
+    ctx.integrate(x, v, (0, -9.8, 0), sc.dt)
+    ctx.pd_solve(x, v, h, sc.mu, sc.lam, sc.iterations, sc.dt)
+    ctx.check_status()
+    xo, vo = oracle.integrate(x0, v0, (0, -9.8, 0), sc.dt)
+    xo, _ = oracle.pd_solve(xo, vo, ri, cap, re.shape[0], oidx, opos, oinv, sc.bulk, h, sc.mu, sc.lam, sc.iterations,
+                            sc.dt)
+    assert rel(x.cpu().numpy(), xo) < 1e-5
+
+
+def test_broken_bonds_reach_the_step_by_step_projection(ctx, oracle):
+    sc, x0, h, _, _ = bar(ctx, oracle, 3.0, 80, seed=6)
+    x, v = t(x0 * np.float32([1.06, 1.0, 1.0])), t(np.zeros_like(x0))
+    ctx.pd_solve(x, v, h, sc.mu, sc.lam, 0, sc.dt, 0.05)  # no iteration: bonds along x break, x stays
+    assert torch.equal(x, t(x0 * np.float32([1.06, 1.0, 1.0])))
+    got = []
+    for whole in (True, False):
+        y, u = x.clone(), v.clone()
+        if whole:
+            ctx.pd_solve(y, u, h, sc.mu, sc.lam, 3, sc.dt)
+        else:
+            ctx.pd_begin(y, h, sc.mu, sc.lam, sc.dt)
+            for _ in range(3):
+                ctx.pd_enforce(y, h, sc.mu, sc.lam, sc.dt)
+            ctx.pd_update_velocity(y, u, sc.dt)
+        got.append((y, u))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    y, u = x.clone(), v.clone()
+    bar(ctx, oracle, 3.0, 80, seed=6)  # the same shape, whole again
+    ctx.pd_solve(y, u, h, sc.mu, sc.lam, 3, sc.dt)
+    ctx.check_status()
+    assert not torch.equal(y, got[0][0])
+
+
+def test_rollout_without_projection(ctx, oracle):
+    sc, x0, h, _, _ = bar(ctx, oracle, 3.0, 80, seed=7)
+    x, v = t(x0), t(np.ones_like(x0))
+    ctx.pd_rollout(x, v, h, sc.mu, sc.lam, 0, sc.dt, steps=3, checkpoint_every=2)
+    gx, gv, gb = ctx.pd_rollout_backward(torch.ones_like(x))
+    x2, v2 = t(x0), t(np.ones_like(x0))
+    for _ in range(3):
+        ctx.integrate(x2, v2, (0.0, -9.8, 0.0), sc.dt)
+    ctx.check_status()
+    assert torch.equal(x, x2) and torch.equal(v, v2)
+    assert torch.equal(gx, torch.ones_like(x)) and float(gb.abs().max()) == 0.0
+    assert rel(gv.cpu().numpy(), np.full(x0.shape, 3 * sc.dt)) < 1e-6
