@@ -46,6 +46,18 @@ bool regrow(T*& p, size_t count)
     return cudaMalloc((void**)&p, sizeof(T) * count) == cudaSuccess;
 }
 
+// Every cell count to zero (the tables or the keys they hold are new), done
+// before anything on any stream can read them.
+int clear_cells(pk_ctx* c)
+{
+    cudaError_t e = cudaMemset(c->counters, 0, 4 * sizeof(int));
+    if (e == cudaSuccess && c->cap_keys > 0) e = cudaMemset(c->cell_cnt, 0, sizeof(int) * ((size_t)c->cap_keys + 1));
+    if (e == cudaSuccess && c->cap_keys > 0)
+        e = cudaMemset(c->blk_cnt, 0, sizeof(int) * ((size_t)(c->cap_keys >> 6) + 2));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e == cudaSuccess ? PK_OK : cuda_fail(c, e, "clearing the cell table");
+}
+
 int ensure_particles(pk_ctx* c, int n)
 {
     if (n <= c->cap_n) return PK_OK;
@@ -55,7 +67,7 @@ int ensure_particles(pk_ctx* c, int n)
               regrow(c->xs_pre, m) && regrow(c->xs0, m) && regrow(c->xa, m) && regrow(c->xb, m) &&
               regrow(c->vs, m) && regrow(c->vv, m) && regrow(c->rho, m) && regrow(c->rcnt, m) &&
               regrow(c->tau, m) && regrow(c->tau_hint, m) && regrow(c->hcnt, m) && regrow(c->items, m + 1) &&
-              regrow(c->nitems, 1) && regrow(c->ovf, m) && regrow(c->ovf_list, m) && regrow(c->tile_cnt, m + 2) &&
+              regrow(c->ovf, m) && regrow(c->ovf_list, m) && regrow(c->tile_cnt, m + 2) &&
               regrow(c->tile_off, m + 2) && regrow(c->tiles, m + m / 128 + 2);
     if (!ok) {
         c->cap_n = 0;
@@ -66,7 +78,8 @@ int ensure_particles(pk_ctx* c, int n)
     if (cudaMemset(c->tau_hint, 0xff, sizeof(unsigned) * m) != cudaSuccess)
         return fail(c, PK_ERR_CUDA, "cudaMemset of the selection pivots failed");
     c->cap_n = n;
-    return PK_OK;
+    // the keys that say which cell counts to clear went with the old arrays
+    return clear_cells(c);
 }
 
 int ensure_rows(pk_ctx* c, long long m)
@@ -115,13 +128,17 @@ long long spill_used(pk_ctx* c, cudaStream_t st, int n = 0, int* offs_n = nullpt
 int ensure_keys(pk_ctx* c, long long nk, int n)
 {
     if (nk > c->cap_keys) {
-        if (!regrow(c->cell_cnt, (size_t)nk + 1) || !regrow(c->cell_start, (size_t)nk + 2)) {
+        const size_t blocks = (size_t)(nk >> 6);
+        if (!regrow(c->cell_cnt, (size_t)nk + 1) || !regrow(c->cell_start, (size_t)nk + 1) ||
+            !regrow(c->blk_cnt, blocks + 2) || !regrow(c->blk_start, blocks + 3)) {
             c->cap_keys = 0;
             return fail(c, PK_ERR_NOMEM, "device allocation of the cell table failed");
         }
         c->cap_keys = nk;
+        const int rc = clear_cells(c);
+        if (rc) return rc;
     }
-    long long parts = std::max(pk::scan_parts_needed(nk + 1), pk::scan_parts_needed(n));
+    long long parts = std::max(pk::scan_parts_needed((nk >> 6) + 2), pk::scan_parts_needed(n));
     if (parts > c->cap_part) {
         if (!regrow(c->scan_part, (size_t)parts)) {
             c->cap_part = 0;
@@ -265,10 +282,13 @@ PK_API int pk_ctx_create(pk_ctx** out, int device)
     c->device = device;
     if (cudaMalloc((void**)&c->d_err, sizeof(int)) != cudaSuccess ||
         cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void**)&c->counters, 4 * sizeof(int)) != cudaSuccess ||
+        cudaMemset(c->counters, 0, 4 * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void**)&c->spill, 2 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMemset(c->spill, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) {
         if (c->d_err) cudaFree(c->d_err);
         if (c->spill) cudaFree(c->spill);
+        if (c->counters) cudaFree(c->counters);
         delete c;
         return PK_ERR_NOMEM;
     }
@@ -289,9 +309,9 @@ PK_API int pk_ctx_destroy(pk_ctx* c)
     void* ptrs[] = {c->d_err, c->perm, c->inv, c->key, c->rank, c->count, c->count_c, c->offs,
                     c->xs_pre, c->xs0, c->xa, c->xb, c->vs, c->vv, c->rho, c->rcnt, c->tau, c->tau_hint, c->pl_y1, c->pl_y2, c->pl_i1, c->pl_yield,
                     c->pl_invF, c->pl_sizes, c->pl_off, c->pl_rest_idx2, c->pl_rest_pos2,
-                    c->hcnt, c->items, c->nitems,
+                    c->hcnt, c->items, c->counters,
                     c->rows, c->hits, c->hpool, c->rpool, c->ovf, c->ovf_list, c->spill, c->tile_cnt,
-                    c->tile_off, c->tiles, c->cell_cnt, c->cell_start, c->scan_part, c->g_rho, c->g_lam,
+                    c->tile_off, c->tiles, c->cell_cnt, c->cell_start, c->blk_cnt, c->blk_start, c->scan_part, c->g_rho, c->g_lam,
                     c->g_dpos, c->g_xold, c->sdf, c->pd_index, c->pd_rest_idx, c->pd_rest_pos,
                     c->pd_alive, c->pd_invK, c->pd_bulk, c->pd_bond, c->pd_raw,
                     c->pd_in_cnt, c->pd_in_off, c->pd_in, c->pd_in_slot, c->h_x, c->h_v, c->pd_ktw, c->pl_mk};

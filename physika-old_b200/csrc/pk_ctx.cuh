@@ -27,7 +27,7 @@ struct pk_ctx {
     int* offs = nullptr;      // exclusive scan of count_c (n + 1)
     int* hcnt = nullptr;      // hits per particle in the hit rows (sorted order)
     int2* items = nullptr;    // list-build work items: sorted ranges sharing one cell
-    int* nitems = nullptr;    // device counter of items (1 int)
+    int* counters = nullptr;  // device: items, occupied blocks of cells, keys the cell counts hold
     float4* xs_pre = nullptr;
     float4* xs0 = nullptr;
     float4* xa = nullptr;
@@ -61,8 +61,10 @@ struct pk_ctx {
 
     // ---- dense cell table (capacity cap_keys entries + 2)
     long long cap_keys = 0;
-    int* cell_cnt = nullptr;
-    int* cell_start = nullptr;
+    int* cell_cnt = nullptr;    // particles per cell: all zero but for the cells of key[0 .. counters[2])
+    int* cell_start = nullptr;  // first sorted slot of every occupied cell (others are not written)
+    int* blk_cnt = nullptr;     // the same per block of 64 consecutive keys
+    int* blk_start = nullptr;   // its exclusive scan
     int* scan_part = nullptr;  // block partials of the scan
     long long cap_part = 0;
 

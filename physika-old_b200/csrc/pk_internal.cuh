@@ -11,7 +11,8 @@
 //                bits 0-29: sorted index j.  Entries with bit31 come first.
 //   rcnt[n]      int2 {#entries with bit31, #entries in the row}
 //   tau[n]       uint2 {float bits of the cap-th smallest distance, its caller id}
-//   cell_cnt / cell_start  dense blocked-Morton cell table (nkeys + 1 / + 2)
+//   cell_cnt / cell_start  dense blocked-Morton cell table (the outside bucket at nkeys)
+//   blk_cnt / blk_start    particles per block of 64 keys and their exclusive scan
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -74,7 +74,8 @@ __device__ __forceinline__ float exact_d2(float4 a, float4 b)
 
 struct BuildArgs {
     const float4* xs;   // positions the list is built on (sorted)
-    const int* start;   // cell starts
+    const int* start;   // starts of the occupied cells
+    const int* count;   // particles per cell
     const int2* items;  // (begin, end) sorted ranges sharing one cell
     const int* nitems;
     Grid g;
@@ -153,8 +154,8 @@ __device__ __forceinline__ int sweep_ranges(const BuildArgs& A, SweepSmem& S, in
     if (lane < 27) {
         const int key = cell_key(A.g, c.x + kOffset27[lane][0], c.y + kOffset27[lane][1], c.z + kOffset27[lane][2]);
         if (key >= 0) {
-            beg = __ldg(A.start + base + key);
-            len = __ldg(A.start + base + key + 1) - beg;
+            beg = __ldg(A.start + base + key);  // not written, and not used, where the cell is empty
+            len = __ldg(A.count + base + key);
         }
     }
     int incl = len;
@@ -888,7 +889,8 @@ int build_rows(pk_ctx* c, int n, const Grid& g, float h, int cap, int row_cap, i
     A.xs = c->xs_pre;
     A.start = c->cell_start;
     A.items = c->items;
-    A.nitems = c->nitems;
+    A.count = c->cell_cnt;
+    A.nitems = c->counters;
     A.g = g;
     A.n = n;
     A.row_cap = row_cap;

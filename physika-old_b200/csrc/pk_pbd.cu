@@ -391,29 +391,32 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     }
 }
 
-// Scene tiles from the cell table: scene s holds the sorted range
-// [start[s K], start[(s+1) K]) (K keys per scene), the particles outside
-// every grid [start[nkeys], n).  One thread per scene.
-__global__ void __launch_bounds__(256) k_tile_count(const int* __restrict__ start, long long scene_keys,
-                                                    int nscenes, long long nkeys, int tile, int* __restrict__ cnt)
+// Scene tiles from the starts of the 64-cell blocks (K of them per scene):
+// scene q holds the sorted range [start[q K], start[(q+1) K]), the particles
+// outside every grid the block past the last.  One thread per scene.
+__device__ __forceinline__ int2 scene_range(const int* start, long long scene_blocks, int nscenes, int q)
+{
+    const long long b = (long long)q * scene_blocks;
+    return make_int2(start[b], start[q < nscenes ? b + scene_blocks : b + 1]);
+}
+__global__ void __launch_bounds__(256) k_tile_count(const int* __restrict__ start, long long scene_blocks,
+                                                    int nscenes, int tile, int* __restrict__ cnt)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q > nscenes) return;
-    const int b = q < nscenes ? start[(long long)q * scene_keys] : start[nkeys];
-    const int e = q < nscenes ? start[(long long)(q + 1) * scene_keys] : start[nkeys + 1];
-    cnt[q] = (e - b + tile - 1) / tile;
+    const int2 r = scene_range(start, scene_blocks, nscenes, q);
+    cnt[q] = (r.y - r.x + tile - 1) / tile;
 }
 
-__global__ void __launch_bounds__(256) k_tile_fill(const int* __restrict__ start, long long scene_keys,
-                                                   int nscenes, long long nkeys, int tile,
-                                                   const int* __restrict__ off, int2* __restrict__ tiles)
+__global__ void __launch_bounds__(256) k_tile_fill(const int* __restrict__ start, long long scene_blocks,
+                                                   int nscenes, int tile, const int* __restrict__ off,
+                                                   int2* __restrict__ tiles)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q > nscenes) return;
-    const int b = q < nscenes ? start[(long long)q * scene_keys] : start[nkeys];
-    const int e = q < nscenes ? start[(long long)(q + 1) * scene_keys] : start[nkeys + 1];
+    const int2 r = scene_range(start, scene_blocks, nscenes, q);
     int o = off[q];
-    for (int a = b; a < e; a += tile) tiles[o++] = make_int2(a, min(a + tile, e));
+    for (int a = r.x; a < r.y; a += tile) tiles[o++] = make_int2(a, min(a + tile, r.y));
 }
 
 // Sorted -> caller order: x, v += (x - x_old)/dt (DP_UpdateVelocity,
@@ -631,10 +634,9 @@ int pbd_fast_solve(pk_ctx* c, int n, const Spiky& k, float mass, int iterations,
     if (persist && c->grid.nscenes > 1) {
         const int ns = c->grid.nscenes;
         const unsigned nb = (unsigned)((ns + 1 + 255) / 256);
-        k_tile_count<<<nb, 256, 0, st>>>(c->cell_start, c->grid.scene_keys, ns, c->grid.nkeys, pb, c->tile_cnt);
+        k_tile_count<<<nb, 256, 0, st>>>(c->blk_start, c->grid.scene_keys >> 6, ns, pb, c->tile_cnt);
         exclusive_scan(c->tile_cnt, ns + 1, c->tile_off, c->scan_part, st);
-        k_tile_fill<<<nb, 256, 0, st>>>(c->cell_start, c->grid.scene_keys, ns, c->grid.nkeys, pb, c->tile_off,
-                                        c->tiles);
+        k_tile_fill<<<nb, 256, 0, st>>>(c->blk_start, c->grid.scene_keys >> 6, ns, pb, c->tile_off, c->tiles);
         T = SceneTiles{c->tiles, c->tile_off + ns + 1};
         launches += 2 + scan_launches();
     }

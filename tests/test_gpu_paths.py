@@ -1,6 +1,7 @@
-"""The branches that sizes and histories take: bond rows too long to be ordered,
-and broken bonds seen by the step-by-step projection.  The oracle is the CPU
-restatement; where two paths of the library must agree, they agree bit for bit."""
+"""The branches that sizes and histories take: consecutive builds on one context,
+bond rows too long to be ordered, and broken bonds seen by the step-by-step
+projection.  The oracle is the CPU restatement; where two paths of the library
+must agree, they agree bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -17,6 +18,24 @@ def t(a, dtype=np.float32):
 
 def rel(a, b):
     return float(np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-30))
+
+
+def test_builds_on_one_context_equal_fresh_ones():
+    # a build clears the cell counts by the keys of the one before it: other
+    # counts, radii, boxes, scenes and particles outside the grid in between
+    rng = np.random.default_rng(3)
+    one = pkhot.Context(0)
+    for n, h, hi, cap in ((3000, 0.0125, 1.0, 60), (40, 0.05, 0.6, 0), (3000, 0.006, 1.3, 40), (1, 0.0125, 1.0, 8),
+                          (9000, 0.02, 2.0, 64), (700, 0.0125, 1.0, 60), (2999, 0.0125, 1.0, 0)):
+        x = (0.4 + rng.uniform(0, 4.5 * h * (n / 1000.0) ** (1 / 3), (n, 3))).astype(np.float32)
+        x[n - n // 9:] += np.float32(3.0)
+        fresh = pkhot.Context(0)
+        a = one.nq_build(t(x), h, (0, 0, 0), (hi,) * 3, cap)
+        b = fresh.nq_build(t(x), h, (0, 0, 0), (hi,) * 3, cap)
+        one.check_status()
+        assert a[2] == b[2] and torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+        fresh.close()
+    one.close()
 
 
 def bar(ctx, oracle, ratio, cap, seed=0):
