@@ -66,17 +66,13 @@ int ensure_particles(pk_ctx* c, int n)
               regrow(c->count, m) && regrow(c->count_c, m) && regrow(c->offs, m + 1) &&
               regrow(c->xs_pre, m) && regrow(c->xs0, m) && regrow(c->xa, m) && regrow(c->xb, m) &&
               regrow(c->vs, m) && regrow(c->vv, m) && regrow(c->rho, m) && regrow(c->rcnt, m) &&
-              regrow(c->tau, m) && regrow(c->tau_hint, m) && regrow(c->hcnt, m) && regrow(c->items, m + 1) &&
-              regrow(c->ovf, m) && regrow(c->ovf_list, m) && regrow(c->tile_cnt, m + 2) &&
+              regrow(c->tau_id, m) && regrow(c->hcnt, m) && regrow(c->items, m + 1) &&
+              regrow(c->ovf, m) && regrow(c->tile_cnt, m + 2) &&
               regrow(c->tile_off, m + 2) && regrow(c->tiles, m + m / 128 + 2);
     if (!ok) {
         c->cap_n = 0;
         return fail(c, PK_ERR_NOMEM, "device allocation of particle scratch failed");
     }
-    // no pivot yet: all ones sits above every distance, so the first selection
-    // takes the plain rounds
-    if (cudaMemset(c->tau_hint, 0xff, sizeof(unsigned) * m) != cudaSuccess)
-        return fail(c, PK_ERR_CUDA, "cudaMemset of the selection pivots failed");
     c->cap_n = n;
     // the keys that say which cell counts to clear went with the old arrays
     return clear_cells(c);
@@ -284,8 +280,8 @@ PK_API int pk_ctx_create(pk_ctx** out, int device)
         cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess ||
         cudaMalloc((void**)&c->counters, 4 * sizeof(int)) != cudaSuccess ||
         cudaMemset(c->counters, 0, 4 * sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void**)&c->spill, 2 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemset(c->spill, 0, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaMalloc((void**)&c->spill, sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemset(c->spill, 0, sizeof(unsigned long long)) != cudaSuccess) {
         if (c->d_err) cudaFree(c->d_err);
         if (c->spill) cudaFree(c->spill);
         if (c->counters) cudaFree(c->counters);
@@ -307,10 +303,10 @@ PK_API int pk_ctx_destroy(pk_ctx* c)
     for (auto& e : c->tune.ev)
         if (e) cudaEventDestroy(e);
     void* ptrs[] = {c->d_err, c->perm, c->inv, c->key, c->rank, c->count, c->count_c, c->offs,
-                    c->xs_pre, c->xs0, c->xa, c->xb, c->vs, c->vv, c->rho, c->rcnt, c->tau, c->tau_hint, c->pl_y1, c->pl_y2, c->pl_i1, c->pl_yield,
+                    c->xs_pre, c->xs0, c->xa, c->xb, c->vs, c->vv, c->rho, c->rcnt, c->tau_id, c->pl_y1, c->pl_y2, c->pl_i1, c->pl_yield,
                     c->pl_invF, c->pl_sizes, c->pl_off, c->pl_rest_idx2, c->pl_rest_pos2,
                     c->hcnt, c->items, c->counters,
-                    c->rows, c->hits, c->hpool, c->rpool, c->ovf, c->ovf_list, c->spill, c->tile_cnt,
+                    c->rows, c->hits, c->hpool, c->rpool, c->ovf, c->spill, c->tile_cnt,
                     c->tile_off, c->tiles, c->cell_cnt, c->cell_start, c->blk_cnt, c->blk_start, c->scan_part, c->g_rho, c->g_lam,
                     c->g_dpos, c->g_xold, c->sdf, c->pd_index, c->pd_rest_idx, c->pd_rest_pos,
                     c->pd_alive, c->pd_invK, c->pd_bulk, c->pd_bond, c->pd_raw,

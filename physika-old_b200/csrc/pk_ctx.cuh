@@ -30,34 +30,32 @@ struct pk_ctx {
     int* counters = nullptr;  // device: items, occupied blocks of cells, keys the cell counts hold
     float4* xs_pre = nullptr;
     float4* xs0 = nullptr;
-    float4* xa = nullptr;
+    float4* xa = nullptr;     // Jacobi iterate; during the build (x, tau's d2) per sorted particle
     float4* xb = nullptr;     // (x, lambda) written by pass A
     float4* vs = nullptr;
     float4* vv = nullptr;     // sorted velocities of the viscosity sweeps
     float* rho = nullptr;
     int2* rcnt = nullptr;
-    uint2* tau = nullptr;
-    unsigned* tau_hint = nullptr;  // caller order: d2 bits of the last frame's tau (selection pivot)
+    int* tau_id = nullptr;    // sorted index that decides a tie at the cap (where xt says so)
 
     // ---- rows (capacity cap_rows entries: row_cap per particle)
     long long cap_rows = 0;
     int* rows = nullptr;      // solver rows: sorted index | flag bits
-    uint2* hits = nullptr;    // hit rows: (sorted index, d2 bits), candidate order
+    int* hits = nullptr;      // hit rows: sorted indices, candidate order (laid out as rows)
     // Entries of a particle past row_cap (hits and solver row alike) go to the
     // spill pool: ovf[s] is the particle's segment, holding round4(count -
-    // row_cap) entries of each array.  spill[0] counts the entries handed out
+    // row_cap) entries of each array.  *spill counts the entries handed out
     // in the last build (also past pool_cap: the size the next build grows the
-    // pool to), spill[1] the particles listed in ovf_list.
+    // pool to).
     long long pool_cap = 0;
     long long pool_need = 0;  // entries the last synchronised build asked for
-    uint2* hpool = nullptr;
+    int* hpool = nullptr;
     int* rpool = nullptr;
     int* tile_cnt = nullptr;  // persistent passes: tiles per scene (n + 2)
     int* tile_off = nullptr;  // their exclusive scan (n + 2; [nscenes + 1] = tiles)
     int2* tiles = nullptr;    // sorted ranges of the tiles (n + n/128 + 2)
     int* ovf = nullptr;       // per sorted particle (valid where its count > row_cap)
-    int* ovf_list = nullptr;  // sorted particles with a spill segment
-    unsigned long long* spill = nullptr;  // 2 device counters
+    unsigned long long* spill = nullptr;  // device counter
 
     // ---- dense cell table (capacity cap_keys entries + 2)
     long long cap_keys = 0;

@@ -10,7 +10,8 @@
 //                bit31: j is in N(i) (i's capped list), bit30: i is in N(j),
 //                bits 0-29: sorted index j.  Entries with bit31 come first.
 //   rcnt[n]      int2 {#entries with bit31, #entries in the row}
-//   tau[n]       uint2 {float bits of the cap-th smallest distance, its caller id}
+//   xa[n]        while the list is built: float4 (position, squared distance of the
+//                cap-th nearest hit), gathered together by the row emission
 //   cell_cnt / cell_start  dense blocked-Morton cell table (the outside bucket at nkeys)
 //   blk_cnt / blk_start    particles per block of 64 keys and their exclusive scan
 #pragma once

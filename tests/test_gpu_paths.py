@@ -1,13 +1,15 @@
-"""The branches that sizes and histories take: consecutive builds on one context,
-bond rows too long to be ordered, and broken bonds seen by the step-by-step
-projection.  The oracle is the CPU restatement; where two paths of the library
-must agree, they agree bit for bit."""
+"""The branches that sizes and histories take: the list build's shared-memory
+stage and what exceeds it, consecutive builds on one context, bond rows too long
+to be ordered, and broken bonds seen by the step-by-step projection.  The oracle
+is the CPU restatement; where two paths of the library must agree, they agree bit
+for bit."""
 import numpy as np
 import pytest
 import torch
 
 import pkhot
 import scenes
+from nbr_util import compare_capped, rows
 
 pytestmark = pytest.mark.gpu
 
@@ -18,6 +20,28 @@ def t(a, dtype=np.float32):
 
 def rel(a, b):
     return float(np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-30))
+
+
+# particles per cell: 104 and 192 are the longest staged rows (25 and 46 per
+# cell), 384 and 640 the staged candidates (19 and 31); 128 the row capacity,
+# or 132 where the call asks for it
+@pytest.mark.parametrize("per_cell", [4, 15, 18, 20, 23, 25, 27, 30, 32, 37, 48, 60])
+@pytest.mark.parametrize("cap,most", [(60, 0), (20, 0), (100, 0), (0, 0), (0, 132)])
+def test_lists_around_the_stage(ctx, oracle, per_cell, cap, most):
+    h = 0.0125
+    n = per_cell * 64
+    x = (0.4 + np.random.default_rng(per_cell).uniform(0, 4 * h, (n, 3))).astype(np.float32)
+    x[1::7] = np.round(x[1::7] / (h / 4)).astype(np.float32) * np.float32(h / 4)  # equal distances too
+    idx, el, _ = ctx.nq_build(t(x), h, (0, 0, 0), (1, 1, 1), cap, max_neighbors=most)
+    ctx.check_status()
+    ri, re = oracle.neighbor_query(x, h, (0, 0, 0), (1, 1, 1), cap)
+    gi, ge = idx.cpu().numpy(), el.cpu().numpy()
+    assert np.array_equal(gi, ri[:n])
+    ga, rb = rows(gi, ge, cap, n), rows(ri, re, cap, n)
+    if cap:
+        assert not compare_capped(x, ga, rb, oracle.dist3, h)
+    else:
+        assert all(np.array_equal(a, b) for a, b in zip(ga, rb))
 
 
 def test_builds_on_one_context_equal_fresh_ones():
