@@ -55,6 +55,15 @@ __host__ __device__ inline long long row_slots(long long n, int row_cap)
     return ((n + 31) & ~31LL) * 4LL * row_quads(row_cap);
 }
 
+// Particles up to which a walk over rows keeps 4 quads in flight per thread
+// instead of one: two blocks of 256 per SM.  Below, a walk is a chain of a
+// row's load latencies; above, the resident warps hide them.  Density and
+// displacement pass, 4 quads against one: 5.0 / 5.3
+// and 7.5 / 7.5 us at 1k particles, 6.8 / 7.2 and 10.2 / 11.0 at 32k, 9.1 / 10.0
+// and 11.4 / 11.8 at 65k; but 18.7 / 20.3 and 16.1 / 17.5 at 152k, 217 / 243 and
+// 185 / 196 at 2M, where the loads in flight cost more warps than they bring.
+constexpr int kDeepMax = 148 * 512;
+
 // Row entry e of sorted particle s (e < its row length): the main array up
 // to the row capacity, then the particle's spill segment.
 struct RowView {

@@ -21,7 +21,8 @@
 
 namespace pk {
 
-// Per-pair constants of the two passes (Spiky kernel, Kernel.h SpikyKernel).
+// Constants of the two passes (Spiky kernel, Kernel.h SpikyKernel); all but
+// inv_h multiply a finished sum, so no pair spends an instruction on them.
 struct PassK {
     float inv_h, cwm, cg, c10g;
 };
@@ -31,6 +32,15 @@ __host__ __device__ inline PassK pass_k(const Spiky& k, float mass)
 }
 constexpr float kEps2 = kEpsilon * kEpsilon;  // r > EPSILON  <=>  r^2 > EPSILON^2
 
+// 1/sqrt of a normal number (the callers clamp from below): one instruction,
+// where rsqrtf also handles denormals.
+__device__ __forceinline__ float rsq(float v)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Pair geometry shared by both passes: r from one reciprocal square root
 // (r = d2 / sqrt(d2); d2 = 0 gives r = 0), 1/r, and d = 1 - r/h clamped at 0,
 // so w = cw d^3 and |grad| = cg d^2 vanish beyond h as in SpikyKernel.
@@ -38,14 +48,11 @@ __device__ __forceinline__ void pair_geom(float dx, float dy, float dz, float in
                                           float& dd)
 {
     d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    ir = rsqrtf(fmaxf(d2, 1e-30f));
+    ir = rsq(fmaxf(d2, 1e-30f));
     dd = fmaxf(fmaf(-(d2 * ir), inv_h, 1.0f), 0.0f);
 }
 
-#ifndef PK_PASS_BLOCK
-#define PK_PASS_BLOCK 256
-#endif
-constexpr int kPassBlock = PK_PASS_BLOCK;  // threads per block of the Jacobi passes
+constexpr int kPassPrefetch = 2;  // row quads a viscosity sweep keeps ahead of the one it works on
 
 // One quad of row entries (16 bytes, streaming: the rows are read once per
 // pass and outgrow L2).
@@ -60,121 +67,21 @@ struct Tail {
     __device__ __forceinline__ int entry(int s, int k) const { return __ldg(rpool + __ldg(ovf + s) + k); }
 };
 
-// Pass A: rho_i and lambda_i over N(i), one thread per particle walking its
-// interleaved row.  Writes xl[s] = (x_i, lambda_i) so pass B gathers a
-// neighbour's position and lambda in one 16-byte load.  sum |grad_j|^2 is taken
-// as sum g_j^2 (|x_ij / r| = 1).
-__global__ void __launch_bounds__(kPassBlock)
-    k_pass_density(const float4* __restrict__ xs, const int* __restrict__ rows,
-                   const int2* __restrict__ rcnt, int row_cap, int n, PassK k_,
-                   float4* __restrict__ xl, float* __restrict__ rho_out, Tail tl)
+// Entry v's position: the flag bits leave with the shift, and the 32-bit byte
+// offset needs no 64-bit arithmetic (rows of 2^28 particles would not fit any
+// memory).
+__device__ __forceinline__ float4 row_pos(const float4* __restrict__ x, int v)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const float4 xi = xs[s];
-    const int na_all = rcnt[s].x, na = min(na_all, row_cap);
-    const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
-    float rho = 0.f, sg = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-    auto pair = [&](int v) {
-        const float4 xj = __ldg(xs + (v & kRowIndexMask));
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        float d2, ir, dd;
-        pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
-        const float dd2 = dd * dd;
-        rho = fmaf(k_.cwm, dd2 * dd, rho);
-        const float g = d2 > kEps2 ? k_.cg * dd2 : 0.0f;
-        const float gi = g * ir;
-        gx = fmaf(gi, dx, gx);
-        gy = fmaf(gi, dy, gy);
-        gz = fmaf(gi, dz, gz);
-        sg = fmaf(g, g, sg);
-    };
-    const int nq = (na + 3) >> 2;
-    int4 nxt = nq > 0 ? row_quad(rq) : make_int4(0, 0, 0, 0);
-    for (int q = 0; q < nq; ++q) {
-        const int4 cur = nxt;
-        if (q + 1 < nq) nxt = row_quad(rq + 32LL * (q + 1));  // next quad in flight
-        const int ent[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (4 * q + k >= na) break;
-            pair(ent[k]);
-        }
-    }
-    for (int e = na; e < na_all; ++e) pair(tl.entry(s, e - na));
-    float l = sg + (gx * gx + gy * gy + gz * gz);
-    l = -(rho - 1000.0f) / (l + 0.1f);  // rest density hard-coded (DensityPBD.cu:87)
-    xl[s] = make_float4(xi.x, xi.y, xi.z, l > 0.0f ? 0.0f : l);
-    if (rho_out != nullptr) rho_out[s] = rho;
+    return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(x) + ((unsigned)v << 4)));
 }
 
-// Pass B: x_i' = x_i + sum over U(i) of m_ij * 10 (x_i - x_j)(lambda_i +
-// lambda_j) grad(r) / r (DensityPBD.cu:158), m_ij = popcount of the two flag
-// bits; one thread per particle.
-__global__ void __launch_bounds__(kPassBlock)
-    k_pass_disp(const float4* __restrict__ xl, const int* __restrict__ rows, const int2* __restrict__ rcnt,
-                int row_cap, int n, PassK k_, float4* __restrict__ xs_out, Tail tl)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const float4 xi = xl[s];
-    const int nu_all = rcnt[s].y, nu = min(nu_all, row_cap);
-    const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    auto pair = [&](int v) {
-        const float mult = (float)__popc((unsigned)v >> 30);
-        const float4 xj = __ldg(xl + (v & kRowIndexMask));
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        float d2, ir, dd;
-        pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
-        const float c = d2 > kEps2 ? mult * (xi.w + xj.w) * (k_.c10g * (dd * dd)) * ir : 0.0f;
-        ax = fmaf(c, dx, ax);
-        ay = fmaf(c, dy, ay);
-        az = fmaf(c, dz, az);
-    };
-    const int nq = (nu + 3) >> 2;
-    int4 nxt = nq > 0 ? row_quad(rq) : make_int4(0, 0, 0, 0);
-    for (int q = 0; q < nq; ++q) {
-        const int4 cur = nxt;
-        if (q + 1 < nq) nxt = row_quad(rq + 32LL * (q + 1));  // next quad in flight
-        const int ent[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (4 * q + k >= nu) break;
-            pair(ent[k]);
-        }
-    }
-    for (int e = nu; e < nu_all; ++e) pair(tl.entry(s, e - nu));
-    xs_out[s] = make_float4(xi.x + ax, xi.y + ay, xi.z + az, 0.f);
-}
-
-// ---- FP32x2 variants of the passes (sm_100 packed FFMA2/FADD2/FMUL2): two
-// row entries per instruction.  Each lane runs its full quads as two entry
-// pairs, then its last partial quad one entry at a time.  The sums run as two
-// interleaved partial sums (even and odd entries of each pair), so the order
-// of additions differs from the one-entry kernels; the arithmetic of each
-// pair term is identical.  d is taken as x_j - x_i (the exact negation of
-// x_i - x_j), so the accumulated gradients and displacements carry the
-// opposite sign and are negated at the end.
-
-#ifndef PK_PASS_F32X2
-#define PK_PASS_F32X2 1
-#endif
-// Row quads each thread keeps in flight ahead of the one it works on.
-#ifndef PK_PASS_PF
-#define PK_PASS_PF 2
-#endif
-constexpr int kPassPrefetch = PK_PASS_PF;
-
-#ifndef PK_PASS_WARPS
-#define PK_PASS_WARPS 0  // resident warps per SM asked of the register allocator (0: none)
-#endif
-template <int BLOCK>
-constexpr int pass_min_blocks()
-{
-    return PK_PASS_WARPS > 0 && PK_PASS_WARPS / (BLOCK / 32) > 0 ? PK_PASS_WARPS / (BLOCK / 32) : 1;
-}
-
+// Both passes, one thread per particle walking its interleaved row, two row
+// entries per packed FP32x2 instruction (sm_100 FFMA2/FADD2/FMUL2): the full
+// quads as two entry pairs, then the last partial quad one entry at a time.
+// The sums run as two interleaved partial sums (even and odd entries of each
+// pair).  d is taken as x_j - x_i (the exact negation of x_i - x_j), so the
+// accumulated gradients and displacements carry the opposite sign and are
+// negated at the end.
 struct Geom2 {
     float2 dx, dy, dz, d2, ir, dd;
 };
@@ -185,84 +92,171 @@ __device__ __forceinline__ void pair_geom2(const float4& a, const float4& b, con
     g.dy = make_float2(a.y - xi.y, b.y - xi.y);
     g.dz = make_float2(a.z - xi.z, b.z - xi.z);
     g.d2 = __ffma2_rn(g.dz, g.dz, __ffma2_rn(g.dy, g.dy, __fmul2_rn(g.dx, g.dx)));
-    g.ir = make_float2(rsqrtf(fmaxf(g.d2.x, 1e-30f)), rsqrtf(fmaxf(g.d2.y, 1e-30f)));
+    g.ir = make_float2(rsq(fmaxf(g.d2.x, 1e-30f)), rsq(fmaxf(g.d2.y, 1e-30f)));
     const float2 t = __ffma2_rn(__fmul2_rn(g.d2, g.ir), make_float2(-inv_h, -inv_h), make_float2(1.0f, 1.0f));
     g.dd = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));
 }
 
-struct DensAcc {
-    float2 rho, sg, gx, gy, gz;
+// Pass A: rho_i and lambda_i over N(i).  sum |grad_j|^2 is taken as sum g_j^2
+// (|x_ij / r| = 1).
+struct DensPass {
+    using Acc = struct {
+        float2 rho, sg, gx, gy, gz;
+    };
+    static __device__ __forceinline__ int entries(const int2& c) { return c.x; }
+    static __device__ __forceinline__ void pair(const float4& a, const float4& b, int, int, const float4& xi,
+                                                const PassK& k_, Acc& s)
+    {
+        Geom2 g;
+        pair_geom2(a, b, xi, k_.inv_h, g);
+        const float2 dd2 = __fmul2_rn(g.dd, g.dd);
+        s.rho = __ffma2_rn(dd2, g.dd, s.rho);
+        const float2 w = make_float2(g.d2.x > kEps2 ? dd2.x : 0.0f, g.d2.y > kEps2 ? dd2.y : 0.0f);
+        const float2 gi = __fmul2_rn(w, g.ir);
+        s.gx = __ffma2_rn(gi, g.dx, s.gx);
+        s.gy = __ffma2_rn(gi, g.dy, s.gy);
+        s.gz = __ffma2_rn(gi, g.dz, s.gz);
+        s.sg = __ffma2_rn(w, w, s.sg);
+    }
+    // One entry into the .x partial sums (the tail of a row).
+    static __device__ __forceinline__ void one(const float4& a, int, const float4& xi, const PassK& k_, Acc& s)
+    {
+        const float dx = a.x - xi.x, dy = a.y - xi.y, dz = a.z - xi.z;
+        float d2, ir, dd;
+        pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
+        const float dd2 = dd * dd;
+        s.rho.x = fmaf(dd2, dd, s.rho.x);
+        const float w = d2 > kEps2 ? dd2 : 0.0f;
+        const float gi = w * ir;
+        s.gx.x = fmaf(gi, dx, s.gx.x);
+        s.gy.x = fmaf(gi, dy, s.gy.x);
+        s.gz.x = fmaf(gi, dz, s.gz.x);
+        s.sg.x = fmaf(w, w, s.sg.x);
+    }
+    // (x_i, lambda_i), so pass B gathers a neighbour's position and lambda in
+    // one 16-byte load.
+    static __device__ __forceinline__ float4 finish(const float4& xi, const PassK& k_, const Acc& a, float* rho_out,
+                                                    int s)
+    {
+        const float rho = k_.cwm * (a.rho.x + a.rho.y), sg = k_.cg * k_.cg * (a.sg.x + a.sg.y);
+        const float gx = k_.cg * (a.gx.x + a.gx.y), gy = k_.cg * (a.gy.x + a.gy.y), gz = k_.cg * (a.gz.x + a.gz.y);
+        // (explicit, so that every instance of the pass rounds alike)
+        float l = fmaf(gz, gz, fmaf(gy, gy, fmaf(gx, gx, sg)));
+        l = -(rho - 1000.0f) / (l + 0.1f);  // rest density hard-coded (DensityPBD.cu:87)
+        if (rho_out != nullptr) rho_out[s] = rho;
+        return make_float4(xi.x, xi.y, xi.z, l > 0.0f ? 0.0f : l);
+    }
 };
 
-__device__ __forceinline__ void dens_pair(const float4& a, const float4& b, const float4& xi, const PassK& k_,
-                                          DensAcc& s)
-{
-    Geom2 g;
-    pair_geom2(a, b, xi, k_.inv_h, g);
-    const float2 dd2 = __fmul2_rn(g.dd, g.dd);
-    s.rho = __ffma2_rn(make_float2(k_.cwm, k_.cwm), __fmul2_rn(dd2, g.dd), s.rho);
-    const float2 gg = __fmul2_rn(make_float2(k_.cg, k_.cg), dd2);
-    const float2 w = make_float2(g.d2.x > kEps2 ? gg.x : 0.0f, g.d2.y > kEps2 ? gg.y : 0.0f);
-    const float2 gi = __fmul2_rn(w, g.ir);
-    s.gx = __ffma2_rn(gi, g.dx, s.gx);
-    s.gy = __ffma2_rn(gi, g.dy, s.gy);
-    s.gz = __ffma2_rn(gi, g.dz, s.gz);
-    s.sg = __ffma2_rn(w, w, s.sg);
-}
-
-// One entry into the .x partial sums (the tail of a row).
-__device__ __forceinline__ void dens_one(const float4& a, const float4& xi, const PassK& k_, DensAcc& s)
-{
-    const float dx = a.x - xi.x, dy = a.y - xi.y, dz = a.z - xi.z;
-    float d2, ir, dd;
-    pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
-    const float dd2 = dd * dd;
-    s.rho.x = fmaf(k_.cwm, dd2 * dd, s.rho.x);
-    const float w = d2 > kEps2 ? k_.cg * dd2 : 0.0f;
-    const float gi = w * ir;
-    s.gx.x = fmaf(gi, dx, s.gx.x);
-    s.gy.x = fmaf(gi, dy, s.gy.x);
-    s.gz.x = fmaf(gi, dz, s.gz.x);
-    s.sg.x = fmaf(w, w, s.sg.x);
-}
-
-__device__ __forceinline__ void density2_particle(int s, const float4* __restrict__ xs,
-                                                  const int* __restrict__ rows, const int2* __restrict__ rcnt,
-                                                  int row_cap, const PassK& k_, float4* __restrict__ xl,
-                                                  float* __restrict__ rho_out, const Tail& tl)
-{
-    const float4 xi = xs[s];
-    const int na_all = rcnt[s].x, na = min(na_all, row_cap);
-    const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
-    DensAcc a{};
-    const int nfull = na >> 2, nq = (na + 3) >> 2;
-    int4 ring[kPassPrefetch];  // ring[k] = quad q + k of the row
-#pragma unroll
-    for (int k = 0; k < kPassPrefetch; ++k) ring[k] = k < nq ? row_quad(rq + 32LL * k) : make_int4(0, 0, 0, 0);
-    for (int q = 0; q < nfull; ++q) {
-        const int4 cur = ring[0];
-#pragma unroll
-        for (int k = 0; k + 1 < kPassPrefetch; ++k) ring[k] = ring[k + 1];
-        if (q + kPassPrefetch < nq) ring[kPassPrefetch - 1] = row_quad(rq + 32LL * (q + kPassPrefetch));
-        const float4 x0 = __ldg(xs + (cur.x & kRowIndexMask)), x1 = __ldg(xs + (cur.y & kRowIndexMask));
-        const float4 x2 = __ldg(xs + (cur.z & kRowIndexMask)), x3 = __ldg(xs + (cur.w & kRowIndexMask));
-        dens_pair(x0, x1, xi, k_, a);
-        dens_pair(x2, x3, xi, k_, a);
+// Pass B: x_i' = x_i + sum over U(i) of m_ij * 10 (x_i - x_j)(lambda_i +
+// lambda_j) grad(r) / r (DensityPBD.cu:158), m_ij the number of flag bits set
+// (1 or 2: 2 exactly when v >= 0xc0000000).
+struct DispPass {
+    using Acc = struct {
+        float2 ax, ay, az;
+    };
+    static __device__ __forceinline__ int entries(const int2& c) { return c.y; }
+    static __device__ __forceinline__ float mult(int v) { return (unsigned)v >= 0xc0000000u ? 2.0f : 1.0f; }
+    static __device__ __forceinline__ void pair(const float4& a, const float4& b, int va, int vb, const float4& xi,
+                                                const PassK& k_, Acc& s)
+    {
+        Geom2 g;
+        pair_geom2(a, b, xi, k_.inv_h, g);
+        const float2 lw = make_float2(xi.w + a.w, xi.w + b.w);
+        const float2 c = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(mult(va), mult(vb)), lw),
+                                               __fmul2_rn(g.dd, g.dd)), g.ir);
+        const float2 cc = make_float2(g.d2.x > kEps2 ? c.x : 0.0f, g.d2.y > kEps2 ? c.y : 0.0f);
+        s.ax = __ffma2_rn(cc, g.dx, s.ax);
+        s.ay = __ffma2_rn(cc, g.dy, s.ay);
+        s.az = __ffma2_rn(cc, g.dz, s.az);
     }
-    const int rest = na - 4 * nfull;
+    static __device__ __forceinline__ void one(const float4& a, int v, const float4& xi, const PassK& k_, Acc& s)
+    {
+        const float dx = a.x - xi.x, dy = a.y - xi.y, dz = a.z - xi.z;
+        float d2, ir, dd;
+        pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
+        const float c = d2 > kEps2 ? mult(v) * (xi.w + a.w) * (dd * dd) * ir : 0.0f;
+        s.ax.x = fmaf(c, dx, s.ax.x);
+        s.ay.x = fmaf(c, dy, s.ay.x);
+        s.az.x = fmaf(c, dz, s.az.x);
+    }
+    static __device__ __forceinline__ float4 finish(const float4& xi, const PassK& k_, const Acc& a, float*, int)
+    {
+        // the sums hold -(displacement): d was x_j - x_i
+        return make_float4(fmaf(-k_.c10g, a.ax.x + a.ax.y, xi.x), fmaf(-k_.c10g, a.ay.x + a.ay.y, xi.y),
+                           fmaf(-k_.c10g, a.az.x + a.az.y, xi.z), 0.f);
+    }
+};
+
+// One particle of a pass.  NQ row quads are loaded together and their
+// neighbours gathered together (4 NQ gathers in flight), with the next NQ quads
+// already on their way; the additions run in row order whatever NQ is.
+template <class Pass, int NQ>
+__device__ __forceinline__ void pass_particle(int s, const float4* __restrict__ xin, const int* __restrict__ rows,
+                                              const int2* __restrict__ rcnt, int row_cap, const PassK& k_,
+                                              float4* __restrict__ xout, float* __restrict__ rho_out, const Tail& tl)
+{
+    const float4 xi = xin[s];
+    const int m_all = Pass::entries(rcnt[s]), m = min(m_all, row_cap);
+    const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
+    typename Pass::Acc a{};
+    const int nfull = m >> 2, nq = (m + 3) >> 2;
+    int4 last;  // the row's partial quad
+    if (NQ == 1) {
+        // two quads ahead of the one worked on
+        int4 r0 = nq > 0 ? row_quad(rq) : make_int4(0, 0, 0, 0);
+        int4 r1 = nq > 1 ? row_quad(rq + 32) : make_int4(0, 0, 0, 0);
+        for (int q = 0; q < nfull; ++q) {
+            const int4 cur = r0;
+            r0 = r1;
+            if (q + 2 < nq) r1 = row_quad(rq + 32LL * (q + 2));
+            const float4 x0 = row_pos(xin, cur.x), x1 = row_pos(xin, cur.y);
+            const float4 x2 = row_pos(xin, cur.z), x3 = row_pos(xin, cur.w);
+            Pass::pair(x0, x1, cur.x, cur.y, xi, k_, a);
+            Pass::pair(x2, x3, cur.z, cur.w, xi, k_, a);
+        }
+        last = r0;
+    } else {
+        last = nq > nfull ? row_quad(rq + 32LL * nfull) : make_int4(0, 0, 0, 0);
+        int4 nxt[NQ];
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) nxt[k] = k < nfull ? row_quad(rq + 32LL * k) : make_int4(0, 0, 0, 0);
+        for (int q = 0; q < nfull; q += NQ) {
+            int4 cur[NQ];
+            float4 x[4 * NQ];
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) cur[k] = nxt[k];
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {  // entries past the row's end read particle 0, unused
+                x[4 * k] = row_pos(xin, cur[k].x);
+                x[4 * k + 1] = row_pos(xin, cur[k].y);
+                x[4 * k + 2] = row_pos(xin, cur[k].z);
+                x[4 * k + 3] = row_pos(xin, cur[k].w);
+            }
+#pragma unroll
+            for (int k = 0; k < NQ; ++k)
+                nxt[k] = q + NQ + k < nfull ? row_quad(rq + 32LL * (q + NQ + k)) : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {
+                if (q + k < nfull) {
+                    Pass::pair(x[4 * k], x[4 * k + 1], cur[k].x, cur[k].y, xi, k_, a);
+                    Pass::pair(x[4 * k + 2], x[4 * k + 3], cur[k].z, cur[k].w, xi, k_, a);
+                }
+            }
+        }
+    }
+    const int rest = m - 4 * nfull;
     if (rest > 0) {
-        const int ent[3] = {ring[0].x, ring[0].y, ring[0].z};
+        const int ent[3] = {last.x, last.y, last.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k)
-            if (k < rest) dens_one(__ldg(xs + (ent[k] & kRowIndexMask)), xi, k_, a);
+            if (k < rest) Pass::one(row_pos(xin, ent[k]), ent[k], xi, k_, a);
     }
-    for (int e = na; e < na_all; ++e) dens_one(__ldg(xs + (tl.entry(s, e - na) & kRowIndexMask)), xi, k_, a);
-    const float rho = a.rho.x + a.rho.y, sg = a.sg.x + a.sg.y;
-    const float gx = a.gx.x + a.gx.y, gy = a.gy.x + a.gy.y, gz = a.gz.x + a.gz.y;
-    float l = sg + (gx * gx + gy * gy + gz * gz);
-    l = -(rho - 1000.0f) / (l + 0.1f);  // rest density hard-coded (DensityPBD.cu:87)
-    xl[s] = make_float4(xi.x, xi.y, xi.z, l > 0.0f ? 0.0f : l);
-    if (rho_out != nullptr) rho_out[s] = rho;
+    for (int e = m; e < m_all; ++e) {
+        const int v = tl.entry(s, e - m);
+        Pass::one(row_pos(xin, v), v, xi, k_, a);
+    }
+    xout[s] = Pass::finish(xi, k_, a, rho_out, s);
 }
 
 // Tiles of the persistent passes: each scene's sorted range (and the range of
@@ -273,121 +267,30 @@ struct SceneTiles {
     const int* count;  // device: number of tiles
 };
 
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, pass_min_blocks<BLOCK>())
-    k_pass_density2(const float4* __restrict__ xs, const int* __restrict__ rows,
-                    const int2* __restrict__ rcnt, int row_cap, int n, PassK k_,
-                    float4* __restrict__ xl, float* __restrict__ rho_out, Tail tl)
+// Row quads per step of a pass: 1 (the most resident warps) where the
+// particles fill the chip, 4 for the small scenes (kDeepMax).
+template <class Pass, int BLOCK, int NQ>
+__global__ void __launch_bounds__(BLOCK)
+    k_pass(const float4* __restrict__ xin, const int* __restrict__ rows, const int2* __restrict__ rcnt, int row_cap,
+           int n, PassK k_, float4* __restrict__ xout, float* __restrict__ rho_out, Tail tl)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) density2_particle(s, xs, rows, rcnt, row_cap, k_, xl, rho_out, tl);
+    if (s < n) pass_particle<Pass, NQ>(s, xin, rows, rcnt, row_cap, k_, xout, rho_out, tl);
 }
 
 // Persistent form: a grid of resident blocks walks the scene tiles.
 // (32 resident warps per SM asked of the register allocator: the tile loop
 // would otherwise take the kernel past 64 registers and a quarter of them)
-template <int BLOCK>
+template <class Pass, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-    k_pass_density2_t(const float4* __restrict__ xs, const int* __restrict__ rows,
-                      const int2* __restrict__ rcnt, int row_cap, int n, PassK k_,
-                      float4* __restrict__ xl, float* __restrict__ rho_out, Tail tl, SceneTiles T)
+    k_pass_t(const float4* __restrict__ xin, const int* __restrict__ rows, const int2* __restrict__ rcnt, int row_cap,
+             int n, PassK k_, float4* __restrict__ xout, float* __restrict__ rho_out, Tail tl, SceneTiles T)
 {
     const int nt = T.tile ? *T.count : (n + BLOCK - 1) / BLOCK;
     for (int t = blockIdx.x; t < nt; t += gridDim.x) {
         const int2 r = T.tile ? T.tile[t] : make_int2(t * BLOCK, min((t + 1) * BLOCK, n));
         const int s = r.x + (int)threadIdx.x;
-        if (s < r.y) density2_particle(s, xs, rows, rcnt, row_cap, k_, xl, rho_out, tl);
-    }
-}
-
-struct DispAcc {
-    float2 ax, ay, az;
-};
-
-__device__ __forceinline__ void disp_pair(const float4& a, const float4& b, int va, int vb, const float4& xi,
-                                          const PassK& k_, DispAcc& s)
-{
-    Geom2 g;
-    pair_geom2(a, b, xi, k_.inv_h, g);
-    const float2 mult = make_float2((float)__popc((unsigned)va >> 30), (float)__popc((unsigned)vb >> 30));
-    const float2 lw = make_float2(xi.w + a.w, xi.w + b.w);
-    const float2 c = __fmul2_rn(__fmul2_rn(__fmul2_rn(mult, lw),
-                                           __fmul2_rn(make_float2(k_.c10g, k_.c10g), __fmul2_rn(g.dd, g.dd))),
-                                g.ir);
-    const float2 cc = make_float2(g.d2.x > kEps2 ? c.x : 0.0f, g.d2.y > kEps2 ? c.y : 0.0f);
-    s.ax = __ffma2_rn(cc, g.dx, s.ax);
-    s.ay = __ffma2_rn(cc, g.dy, s.ay);
-    s.az = __ffma2_rn(cc, g.dz, s.az);
-}
-
-__device__ __forceinline__ void disp_one(const float4& a, int v, const float4& xi, const PassK& k_, DispAcc& s)
-{
-    const float mult = (float)__popc((unsigned)v >> 30);
-    const float dx = a.x - xi.x, dy = a.y - xi.y, dz = a.z - xi.z;
-    float d2, ir, dd;
-    pair_geom(dx, dy, dz, k_.inv_h, d2, ir, dd);
-    const float c = d2 > kEps2 ? mult * (xi.w + a.w) * (k_.c10g * (dd * dd)) * ir : 0.0f;
-    s.ax.x = fmaf(c, dx, s.ax.x);
-    s.ay.x = fmaf(c, dy, s.ay.x);
-    s.az.x = fmaf(c, dz, s.az.x);
-}
-
-__device__ __forceinline__ void disp2_particle(int s, const float4* __restrict__ xl, const int* __restrict__ rows,
-                                               const int2* __restrict__ rcnt, int row_cap, const PassK& k_,
-                                               float4* __restrict__ xs_out, const Tail& tl)
-{
-    const float4 xi = xl[s];
-    const int nu_all = rcnt[s].y, nu = min(nu_all, row_cap);
-    const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
-    DispAcc a{};
-    const int nfull = nu >> 2, nq = (nu + 3) >> 2;
-    int4 ring[kPassPrefetch];  // ring[k] = quad q + k of the row
-#pragma unroll
-    for (int k = 0; k < kPassPrefetch; ++k) ring[k] = k < nq ? row_quad(rq + 32LL * k) : make_int4(0, 0, 0, 0);
-    for (int q = 0; q < nfull; ++q) {
-        const int4 cur = ring[0];
-#pragma unroll
-        for (int k = 0; k + 1 < kPassPrefetch; ++k) ring[k] = ring[k + 1];
-        if (q + kPassPrefetch < nq) ring[kPassPrefetch - 1] = row_quad(rq + 32LL * (q + kPassPrefetch));
-        const float4 x0 = __ldg(xl + (cur.x & kRowIndexMask)), x1 = __ldg(xl + (cur.y & kRowIndexMask));
-        const float4 x2 = __ldg(xl + (cur.z & kRowIndexMask)), x3 = __ldg(xl + (cur.w & kRowIndexMask));
-        disp_pair(x0, x1, cur.x, cur.y, xi, k_, a);
-        disp_pair(x2, x3, cur.z, cur.w, xi, k_, a);
-    }
-    const int rest = nu - 4 * nfull;
-    if (rest > 0) {
-        const int ent[3] = {ring[0].x, ring[0].y, ring[0].z};
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k < rest) disp_one(__ldg(xl + (ent[k] & kRowIndexMask)), ent[k], xi, k_, a);
-    }
-    for (int e = nu; e < nu_all; ++e) {
-        const int v = tl.entry(s, e - nu);
-        disp_one(__ldg(xl + (v & kRowIndexMask)), v, xi, k_, a);
-    }
-    // the sums hold -(displacement): d was x_j - x_i
-    xs_out[s] = make_float4(xi.x - (a.ax.x + a.ax.y), xi.y - (a.ay.x + a.ay.y), xi.z - (a.az.x + a.az.y), 0.f);
-}
-
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, pass_min_blocks<BLOCK>())
-    k_pass_disp2(const float4* __restrict__ xl, const int* __restrict__ rows, const int2* __restrict__ rcnt,
-                 int row_cap, int n, PassK k_, float4* __restrict__ xs_out, Tail tl)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) disp2_particle(s, xl, rows, rcnt, row_cap, k_, xs_out, tl);
-}
-
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-    k_pass_disp2_t(const float4* __restrict__ xl, const int* __restrict__ rows, const int2* __restrict__ rcnt,
-                   int row_cap, int n, PassK k_, float4* __restrict__ xs_out, Tail tl, SceneTiles T)
-{
-    const int nt = T.tile ? *T.count : (n + BLOCK - 1) / BLOCK;
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int2 r = T.tile ? T.tile[t] : make_int2(t * BLOCK, min((t + 1) * BLOCK, n));
-        const int s = r.x + (int)threadIdx.x;
-        if (s < r.y) disp2_particle(s, xl, rows, rcnt, row_cap, k_, xs_out, tl);
+        if (s < r.y) pass_particle<Pass, 1>(s, xin, rows, rcnt, row_cap, k_, xout, rho_out, tl);
     }
 }
 
@@ -563,21 +466,20 @@ static void by_block(int block, Args&&... args)
     else
         Launch<256>::run(args...);
 }
-template <int B>
-struct LaunchDensity {
-    static void run(unsigned nb, cudaStream_t st, const float4* cur, const int* rows, const int2* rcnt, int row_cap,
-                    int n, PassK pk, float4* xl, float* rho, Tail tl)
-    {
-        k_pass_density2<B><<<nb, B, 0, st>>>(cur, rows, rcnt, row_cap, n, pk, xl, rho, tl);
-    }
-};
-template <int B>
-struct LaunchDisp {
-    static void run(unsigned nb, cudaStream_t st, const float4* xl, const int* rows, const int2* rcnt, int row_cap,
-                    int n, PassK pk, float4* out, Tail tl)
-    {
-        k_pass_disp2<B><<<nb, B, 0, st>>>(xl, rows, rcnt, row_cap, n, pk, out, tl);
-    }
+template <class Pass>
+struct LaunchPass {
+    template <int B>
+    struct At {
+        static void run(unsigned nb, cudaStream_t st, const float4* cur, const int* rows, const int2* rcnt,
+                        int row_cap, int n, PassK pk, float4* out, float* rho, Tail tl)
+        {
+            if (n <= kDeepMax)
+                k_pass<Pass, 64, 4><<<(unsigned)((n + 63) / 64), 64, 0, st>>>(cur, rows, rcnt, row_cap, n, pk, out,
+                                                                            rho, tl);
+            else
+                k_pass<Pass, B, 1><<<nb, B, 0, st>>>(cur, rows, rcnt, row_cap, n, pk, out, rho, tl);
+        }
+    };
 };
 // Resident blocks per SM of a persistent pass kernel (one query per shape).
 template <class K>
@@ -589,23 +491,17 @@ static int resident_blocks(K kernel, int block)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
     return std::max(1, per_sm) * std::max(1, sms);
 }
-template <int B>
-struct LaunchDensityT {
-    static void run(unsigned, cudaStream_t st, const float4* cur, const int* rows, const int2* rcnt, int row_cap,
-                    int n, PassK pk, float4* xl, float* rho, Tail tl, SceneTiles T)
-    {
-        static const int grid = resident_blocks(k_pass_density2_t<B>, B);
-        k_pass_density2_t<B><<<grid, B, 0, st>>>(cur, rows, rcnt, row_cap, n, pk, xl, rho, tl, T);
-    }
-};
-template <int B>
-struct LaunchDispT {
-    static void run(unsigned, cudaStream_t st, const float4* xl, const int* rows, const int2* rcnt, int row_cap,
-                    int n, PassK pk, float4* out, Tail tl, SceneTiles T)
-    {
-        static const int grid = resident_blocks(k_pass_disp2_t<B>, B);
-        k_pass_disp2_t<B><<<grid, B, 0, st>>>(xl, rows, rcnt, row_cap, n, pk, out, tl, T);
-    }
+template <class Pass>
+struct LaunchPassT {
+    template <int B>
+    struct At {
+        static void run(unsigned, cudaStream_t st, const float4* cur, const int* rows, const int2* rcnt, int row_cap,
+                        int n, PassK pk, float4* out, float* rho, Tail tl, SceneTiles T)
+        {
+            static const int grid = resident_blocks(k_pass_t<Pass, B>, B);
+            k_pass_t<Pass, B><<<grid, B, 0, st>>>(cur, rows, rcnt, row_cap, n, pk, out, rho, tl, T);
+        }
+    };
 };
 template <int B>
 struct LaunchVisc {
@@ -629,7 +525,7 @@ int pbd_fast_solve(pk_ctx* c, int n, const Spiky& k, float mass, int iterations,
     const Tail tl{c->rpool, c->ovf};
     // resident-grid passes (an autotuner shape): scene tiles of batched frames
     // from the cell table
-    const bool persist = PK_PASS_F32X2 && c->tune.persist;
+    const bool persist = c->tune.persist;
     SceneTiles T{nullptr, nullptr};
     if (persist && c->grid.nscenes > 1) {
         const int ns = c->grid.nscenes;
@@ -645,24 +541,20 @@ int pbd_fast_solve(pk_ctx* c, int n, const Spiky& k, float mass, int iterations,
     for (int it = 0; it < iterations; ++it) {
         const bool last = it == iterations - 1;
         prof_begin(c, PK_PROF_DENSITY, st);
+        float* const rho = last ? c->rho : nullptr;
         if (persist)
-            by_block<LaunchDensityT>(pb, nbp, st, cur, c->rows, c->rcnt, c->row_cap, n, pk, c->xb,
-                                     last ? c->rho : nullptr, tl, T);
-        else if (PK_PASS_F32X2)
-            by_block<LaunchDensity>(pb, nbp, st, cur, c->rows, c->rcnt, c->row_cap, n, pk, c->xb,
-                                    last ? c->rho : nullptr, tl);
+            by_block<LaunchPassT<DensPass>::At>(pb, nbp, st, cur, c->rows, c->rcnt, c->row_cap, n, pk, c->xb, rho, tl,
+                                                T);
         else
-            k_pass_density<<<(n + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(
-                cur, c->rows, c->rcnt, c->row_cap, n, pk, c->xb, last ? c->rho : nullptr, tl);
+            by_block<LaunchPass<DensPass>::At>(pb, nbp, st, cur, c->rows, c->rcnt, c->row_cap, n, pk, c->xb, rho, tl);
         prof_end(c, PK_PROF_DENSITY, st);
         prof_begin(c, PK_PROF_DISP, st);
         if (persist)
-            by_block<LaunchDispT>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk, c->xa, tl, T);
-        else if (PK_PASS_F32X2)
-            by_block<LaunchDisp>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk, c->xa, tl);
+            by_block<LaunchPassT<DispPass>::At>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk, c->xa,
+                                                (float*)nullptr, tl, T);
         else
-            k_pass_disp<<<(n + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(c->xb, c->rows, c->rcnt,
-                                                                                 c->row_cap, n, pk, c->xa, tl);
+            by_block<LaunchPass<DispPass>::At>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk, c->xa,
+                                               (float*)nullptr, tl);
         prof_end(c, PK_PROF_DISP, st);
         cur = c->xa;
         launches += 2;
@@ -707,10 +599,10 @@ int pbd_replay_solve(pk_ctx* c, int n, const Spiky& k, float mass, int iteration
     const PassK pk = pass_k(k, mass);
     const Tail tl{c->rpool, c->ovf};  // unused: the rollout's rows fit their capacity
     for (int it = 0; it < iterations; ++it) {
-        by_block<LaunchDensity>(pb, nbp, st, ys + (size_t)it * n, c->rows, c->rcnt, c->row_cap, n, pk, c->xb,
-                                nullptr, tl);
-        by_block<LaunchDisp>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk, ys + (size_t)(it + 1) * n,
-                             tl);
+        by_block<LaunchPass<DensPass>::At>(pb, nbp, st, ys + (size_t)it * n, c->rows, c->rcnt, c->row_cap, n, pk, c->xb,
+                                           (float*)nullptr, tl);
+        by_block<LaunchPass<DispPass>::At>(pb, nbp, st, c->xb, c->rows, c->rcnt, c->row_cap, n, pk,
+                                           ys + (size_t)(it + 1) * n, (float*)nullptr, tl);
     }
     k_finish<<<nb1, 256, 0, st>>>(ys + (size_t)iterations * n, ys, c->vs, c->rho, c->inv, n, dt, x, v, nullptr);
     return 2 * iterations + 1;

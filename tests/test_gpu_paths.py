@@ -1,8 +1,8 @@
 """The branches that sizes and histories take: the list build's shared-memory
-stage and what exceeds it, consecutive builds on one context, bond rows too long
-to be ordered, and broken bonds seen by the step-by-step projection.  The oracle
-is the CPU restatement; where two paths of the library must agree, they agree bit
-for bit."""
+stage and what exceeds it, consecutive builds on one context, the two forms of
+a row walk (a few quads or one in flight), bond rows too long to be ordered, and
+broken bonds seen by the step-by-step projection.  The oracle is the CPU
+restatement; where two paths of the library must agree, they agree bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -60,6 +60,30 @@ def test_builds_on_one_context_equal_fresh_ones():
         assert a[2] == b[2] and torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
         fresh.close()
     one.close()
+
+
+@pytest.mark.parametrize("viscosity", [0.0])
+def test_row_walks_of_small_and_large_scenes_agree(viscosity):
+    # each scene alone keeps several quads per thread in flight, both together
+    # (77,788 particles) one: the same sums in the same order
+    ctx = pkhot.Context(0)
+    a = scenes.dam_break_small(seed=1, n_side=1)
+    xs = [scenes.lattice(40, 32, 32, a.spacing, 0.1, 5), scenes.lattice(36, 33, 31, a.spacing, 0.1, 6)]
+    ctx.boundary_set_box(a.lo, a.hi, a.sdf_spacing, True)
+    prm = pkhot.pbf_params(pkhot.nq_params(a.radius, a.lo, a.hi, a.cap),
+                           pkhot.pbd_params(a.radius, a.spacing, 1000.0, 3, a.dt), a.gravity, viscosity=viscosity)
+    vs = [np.random.default_rng(k).normal(0, 0.05, x.shape).astype(np.float32) for k, x in enumerate(xs)]
+    off = np.cumsum([0] + [x.shape[0] for x in xs]).astype(np.int32)
+    xb, vb = t(np.concatenate(xs)), t(np.concatenate(vs))
+    for _ in range(2):
+        ctx.pbf_step_batched(xb, vb, t(off, np.int32), prm)
+    for k in range(2):
+        x, v = t(xs[k]), t(vs[k])
+        for _ in range(2):
+            ctx.pbf_step(x, v, prm)
+        assert torch.equal(x, xb[off[k]:off[k + 1]]) and torch.equal(v, vb[off[k]:off[k + 1]])
+    ctx.check_status()
+    ctx.close()
 
 
 def bar(ctx, oracle, ratio, cap, seed=0):
