@@ -158,6 +158,24 @@ int ensure_generic(pk_ctx* c, int n)
     return PK_OK;
 }
 
+int ensure_viscosity(pk_ctx* c, int n, long long entries, int iterations)
+{
+    if (4LL * n > c->g_quads_cap) {
+        if (!regrow(c->g_quads, 4 * (size_t)n)) {
+            c->g_quads_cap = 0;
+            return fail(c, PK_ERR_NOMEM, "device allocation of viscosity scratch failed");
+        }
+        c->g_quads_cap = 4LL * n;
+    }
+    if (iterations > 1 && entries > c->g_w_cap) {
+        // without this one the sweeps form the weights again
+        const long long want = entries + entries / 8;
+        c->g_w_cap = regrow(c->g_w, (size_t)want) ? want : 0;
+        if (c->g_w_cap == 0) cudaGetLastError();
+    }
+    return PK_OK;
+}
+
 // Entries per particle kept in the main hit and solver rows: 128, or 2 cap
 // for a larger cap; a dynamic list, whose solver rows hold every hit, 192 or
 // its max_neighbors (a multiple of 4).  Longer rows continue in the spill
@@ -308,7 +326,7 @@ PK_API int pk_ctx_destroy(pk_ctx* c)
                     c->hcnt, c->items, c->counters,
                     c->rows, c->hits, c->hpool, c->rpool, c->ovf, c->spill, c->tile_cnt,
                     c->tile_off, c->tiles, c->cell_cnt, c->cell_start, c->blk_cnt, c->blk_start, c->scan_part, c->g_rho, c->g_lam,
-                    c->g_dpos, c->g_xold, c->sdf, c->pd_index, c->pd_rest_idx, c->pd_rest_pos,
+                    c->g_dpos, c->g_xold, c->g_quads, c->g_w, c->sdf, c->pd_index, c->pd_rest_idx, c->pd_rest_pos,
                     c->pd_alive, c->pd_invK, c->pd_bulk, c->pd_bond, c->pd_raw,
                     c->pd_in_cnt, c->pd_in_off, c->pd_in, c->pd_in_slot, c->h_x, c->h_v, c->pd_ktw, c->pl_mk};
     pk::pd_work_release(c);
@@ -1083,7 +1101,7 @@ PK_API int pk_viscosity(pk_ctx* c, const float* x, float* v, int n, const int* i
     if (rc) return rc;
     if (n > 0 && (!x || !v)) return fail(c, PK_ERR_ARG, "null positions or velocities");
     cudaSetDevice(c->device);
-    if ((rc = ensure_generic(c, n))) return rc;
+    if ((rc = ensure_viscosity(c, n, cap > 0 ? (long long)n * cap : total, iterations))) return rc;
     c->launches = pk::viscosity_generic(c, x, v, n, index, elements, cap, total, viscosity, smoothing_length,
                                         iterations, dt, (cudaStream_t)stream);
     return check_launch(c, "pk_viscosity");

@@ -72,6 +72,12 @@ struct pk_ctx {
     float* g_lam = nullptr;
     float* g_dpos = nullptr;  // 3 per particle
     float* g_xold = nullptr;  // 3 per particle
+    // pk_viscosity: 4 packed arrays of n (positions, v_old and two iterates),
+    // and the list's weights where they fit
+    float4* g_quads = nullptr;
+    long long g_quads_cap = 0;
+    float* g_w = nullptr;
+    long long g_w_cap = 0;
     // device copies of the caller's host arrays (pk_pbf_step_host)
     float* h_x = nullptr;  // 3 per particle
     float* h_v = nullptr;  // 3 per particle

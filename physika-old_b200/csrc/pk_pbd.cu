@@ -52,8 +52,6 @@ __device__ __forceinline__ void pair_geom(float dx, float dy, float dz, float in
     dd = fmaxf(fmaf(-(d2 * ir), inv_h, 1.0f), 0.0f);
 }
 
-constexpr int kPassPrefetch = 2;  // row quads a viscosity sweep keeps ahead of the one it works on
-
 // One quad of row entries (16 bytes, streaming: the rows are read once per
 // pass and outgrow L2).
 __device__ __forceinline__ int4 row_quad(const int4* p) { return __ldcs(p); }
@@ -367,53 +365,128 @@ __global__ void __launch_bounds__(256)
 
 // One K_ApplyViscosity sweep over N(i) (the rows' first |N(i)| entries):
 // v_i = v_old,i/(1+b) + (sum w v_j / sum w) b/(1+b); b = 0 and sum w = 1 when
-// sum w < EPSILON.
-template <int BLOCK>
+// sum w < EPSILON.  The weights depend on the positions alone, which no sweep
+// moves: the first sweep (kFirst) forms them, keeps them in wrow, laid out as
+// the rows, and their sum in vold's fourth value; the others read them, 4
+// bytes per entry in place of a 16-byte gather and the pair's geometry.  NQ as
+// in the Jacobi passes.  Bound by L1 as they are: 152k particles, 22 us a sweep
+// after a first of 35, where forming the weights in each took 36.
+__device__ __forceinline__ float4 visc_mix(const float4& vo, float sx, float sy, float sz, float b, float t)
+{
+    // every rounding explicit: the sweeps over rows and over lists agree
+    const float d = 1.0f + b;
+    return make_float4(__fadd_rn(__fdiv_rn(vo.x, d), __fdiv_rn(__fmul_rn(__fdiv_rn(sx, t), b), d)),
+                       __fadd_rn(__fdiv_rn(vo.y, d), __fdiv_rn(__fmul_rn(__fdiv_rn(sy, t), b), d)),
+                       __fadd_rn(__fdiv_rn(vo.z, d), __fdiv_rn(__fmul_rn(__fdiv_rn(sz, t), b), d)), 0.f);
+}
+template <int BLOCK, int NQ, bool kFirst>
 __global__ void __launch_bounds__(BLOCK)
-    k_pass_visc(const float4* __restrict__ xs, const float4* __restrict__ vin, const float4* __restrict__ vold,
-                const int* __restrict__ rows, const int2* __restrict__ rcnt, int row_cap, int n, ViscK k_,
-                float4* __restrict__ vout, Tail tl)
+    k_pass_visc(const float4* __restrict__ xs, const float4* __restrict__ vin, float4* __restrict__ vold,
+                const int* __restrict__ rows, float* __restrict__ wrow, const int2* __restrict__ rcnt, int row_cap,
+                int n, ViscK k_, float4* __restrict__ vout, Tail tl)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const float4 xi = xs[s];
     const int na_all = rcnt[s].x, na = min(na_all, row_cap);
     const int4* rq = reinterpret_cast<const int4*>(rows + row_slot(s, 0, row_cap));
-    float tw = 0.f, dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
-    auto pair = [&](int v) {
-        const int j = v & kRowIndexMask;
-        const float4 xj = __ldg(xs + j);
-        const float4 vj = __ldg(vin + j);
+    float4* wq = reinterpret_cast<float4*>(wrow + row_slot(s, 0, row_cap));
+    float4 vo = vold[s];
+    // one partial sum per place in a quad, as pk_viscosity sums a caller's
+    // list over 4 lanes: both give the same velocities for the same list
+    float tw4[4] = {0.f, 0.f, 0.f, 0.f}, az[4] = {0.f, 0.f, 0.f, 0.f};
+    float2 axy[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+    auto weight = [&](const float4& xj) {
         float d2, ir, dd;
         pair_geom(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, k_.inv_h, d2, ir, dd);
-        const float w = d2 > kEps2 ? k_.cw * dd : 0.0f;
-        tw += w;
-        dx_ = fmaf(w, vj.x, dx_);
-        dy_ = fmaf(w, vj.y, dy_);
-        dz_ = fmaf(w, vj.z, dz_);
+        return d2 > kEps2 ? k_.cw * dd : 0.0f;
     };
-    const int nq = (na + 3) >> 2;
-    int4 ring[kPassPrefetch];  // ring[k] = quad q + k of the row
+    auto add = [&](int k, float w, const float4& vj) {
+        if (kFirst) tw4[k] += w;
+        axy[k] = __ffma2_rn(make_float2(w, w), make_float2(vj.x, vj.y), axy[k]);
+        az[k] = fmaf(w, vj.z, az[k]);
+    };
+    const int nq = (na + 3) >> 2, nfull = na >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    int4 nxt[NQ];
+    float4 wn[NQ];
 #pragma unroll
-    for (int k = 0; k < kPassPrefetch; ++k) ring[k] = k < nq ? row_quad(rq + 32LL * k) : make_int4(0, 0, 0, 0);
-    for (int q = 0; q < nq; ++q) {
-        const int4 cur = ring[0];
+    for (int k = 0; k < NQ; ++k) {
+        nxt[k] = k < nq ? row_quad(rq + 32LL * k) : make_int4(0, 0, 0, 0);
+        wn[k] = !kFirst && k < nq ? __ldcs(wq + 32LL * k) : zero;
+    }
+    int q = 0;
+    for (; q + NQ <= nfull; q += NQ) {
+        int4 cur[NQ];
+        float4 w[NQ], v[4 * NQ], x[kFirst ? 4 * NQ : 1];
 #pragma unroll
-        for (int k = 0; k + 1 < kPassPrefetch; ++k) ring[k] = ring[k + 1];
-        if (q + kPassPrefetch < nq) ring[kPassPrefetch - 1] = row_quad(rq + 32LL * (q + kPassPrefetch));
-        const int ent[4] = {cur.x, cur.y, cur.z, cur.w};
+        for (int k = 0; k < NQ; ++k) {
+            cur[k] = nxt[k];
+            w[k] = wn[k];
+            v[4 * k] = row_pos(vin, cur[k].x);
+            v[4 * k + 1] = row_pos(vin, cur[k].y);
+            v[4 * k + 2] = row_pos(vin, cur[k].z);
+            v[4 * k + 3] = row_pos(vin, cur[k].w);
+            if (kFirst) {
+                x[4 * k] = row_pos(xs, cur[k].x);
+                x[4 * k + 1] = row_pos(xs, cur[k].y);
+                x[4 * k + 2] = row_pos(xs, cur[k].z);
+                x[4 * k + 3] = row_pos(xs, cur[k].w);
+            }
+        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (4 * q + k >= na) break;
-            pair(ent[k]);
+        for (int k = 0; k < NQ; ++k) {
+            const int qn = q + NQ + k;
+            nxt[k] = qn < nq ? row_quad(rq + 32LL * qn) : make_int4(0, 0, 0, 0);
+            if (!kFirst) wn[k] = qn < nq ? __ldcs(wq + 32LL * qn) : zero;
+        }
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            if (kFirst) {
+                w[k] = make_float4(weight(x[4 * k]), weight(x[4 * k + 1]), weight(x[4 * k + 2]), weight(x[4 * k + 3]));
+                __stcs(wq + 32LL * (q + k), w[k]);
+            }
+            add(0, w[k].x, v[4 * k]);
+            add(1, w[k].y, v[4 * k + 1]);
+            add(2, w[k].z, v[4 * k + 2]);
+            add(3, w[k].w, v[4 * k + 3]);
         }
     }
-    for (int e = na; e < na_all; ++e) pair(tl.entry(s, e - na));
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {  // the quads left, the last of them partial
+        const int left = na - 4 * (q + k);
+        if (left <= 0) break;
+        const int ent[4] = {nxt[k].x, nxt[k].y, nxt[k].z, nxt[k].w};
+        float w[4] = {wn[k].x, wn[k].y, wn[k].z, wn[k].w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (kFirst) w[u] = u < left ? weight(row_pos(xs, ent[u])) : 0.f;
+            if (u < left) add(u, w[u], row_pos(vin, ent[u]));
+        }
+        if (kFirst) __stcs(wq + 32LL * (q + k), make_float4(w[0], w[1], w[2], w[3]));
+    }
+    for (int e = na; e < na_all; ++e) {
+        // entry e's place in its quad, without indexing the sums
+        const int v = tl.entry(s, e - na);
+        const float w = weight(row_pos(xs, v));
+        const float4 vj = row_pos(vin, v);
+        const int place = e & 3;
+        if (place == 0) add(0, w, vj);
+        if (place == 1) add(1, w, vj);
+        if (place == 2) add(2, w, vj);
+        if (place == 3) add(3, w, vj);
+    }
+    auto four = [](float a, float b, float c, float d) { return (a + c) + (b + d); };
+    const float sx = four(axy[0].x, axy[1].x, axy[2].x, axy[3].x), sy = four(axy[0].y, axy[1].y, axy[2].y, axy[3].y);
+    const float sz = four(az[0], az[1], az[2], az[3]);
+    float tw = vo.w;
+    if (kFirst) {
+        tw = four(tw4[0], tw4[1], tw4[2], tw4[3]);
+        vold[s].w = tw;
+    }
     const float b = tw < kEpsilon ? 0.0f : k_.b;
     const float t = tw < kEpsilon ? 1.0f : tw;
-    const float4 vo = vold[s];
-    vout[s] = make_float4(vo.x / (1.0f + b) + dx_ / t * b / (1.0f + b), vo.y / (1.0f + b) + dy_ / t * b / (1.0f + b),
-                          vo.z / (1.0f + b) + dz_ / t * b / (1.0f + b), 0.f);
+    vout[s] = visc_mix(vo, sx, sy, sz, b, t);
 }
 
 // Sorted -> caller order with the velocity given: x, v, outDensity (one
@@ -505,10 +578,18 @@ struct LaunchPassT {
 };
 template <int B>
 struct LaunchVisc {
-    static void run(unsigned nb, cudaStream_t st, const float4* xs, const float4* vin, const float4* vold,
-                    const int* rows, const int2* rcnt, int row_cap, int n, ViscK vk, float4* vout, Tail tl)
+    static void run(unsigned nb, cudaStream_t st, bool first, const float4* xs, const float4* vin, float4* vold,
+                    const int* rows, float* wrow, const int2* rcnt, int row_cap, int n, ViscK vk, float4* vout, Tail tl)
     {
-        k_pass_visc<B><<<nb, B, 0, st>>>(xs, vin, vold, rows, rcnt, row_cap, n, vk, vout, tl);
+        const unsigned nd = (unsigned)((n + 63) / 64);
+        if (n <= kDeepMax && first)
+            k_pass_visc<64, 2, true><<<nd, 64, 0, st>>>(xs, vin, vold, rows, wrow, rcnt, row_cap, n, vk, vout, tl);
+        else if (n <= kDeepMax)
+            k_pass_visc<64, 4, false><<<nd, 64, 0, st>>>(xs, vin, vold, rows, wrow, rcnt, row_cap, n, vk, vout, tl);
+        else if (first)
+            k_pass_visc<B, 1, true><<<nb, B, 0, st>>>(xs, vin, vold, rows, wrow, rcnt, row_cap, n, vk, vout, tl);
+        else
+            k_pass_visc<B, 2, false><<<nb, B, 0, st>>>(xs, vin, vold, rows, wrow, rcnt, row_cap, n, vk, vout, tl);
     }
 };
 
@@ -569,7 +650,9 @@ int pbd_fast_solve(pk_ctx* c, int n, const Spiky& k, float mass, int iterations,
         float4* vin = c->vv;
         float4* vout = c->xb;
         for (int t = 0; t < vis_iterations; ++t) {
-            by_block<LaunchVisc>(pb, nbp, st, cur, vin, c->vs, c->rows, c->rcnt, c->row_cap, n, vk, vout, tl);
+            // the hit rows are not needed any more: their place holds the weights
+            by_block<LaunchVisc>(pb, nbp, st, t == 0, cur, vin, c->vs, c->rows, reinterpret_cast<float*>(c->hits),
+                                 c->rcnt, c->row_cap, n, vk, vout, tl);
             float4* tmp = vin;
             vin = vout;
             vout = tmp;
@@ -641,24 +724,58 @@ __device__ __forceinline__ bool valid_id(int j, int n, int* err)
     return false;
 }
 
+// Sums over a caller's list: G lanes per particle read G consecutive entries
+// where a lane per particle read one entry of each of 32 rows.
+struct ListLane {
+    int i, sub, m;
+    long long at;
+    bool valid;
+};
+template <int G>
+__device__ __forceinline__ ListLane list_lane(const int* index, int cap, long long total, int n)
+{
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    ListLane L;
+    L.i = (int)(gid / G);
+    L.sub = (int)(gid % G);
+    L.valid = L.i < n;
+    if (!L.valid) L.i = n - 1;
+    L.m = L.valid ? nb_size(index, cap, total, n, L.i) : 0;
+    L.at = nb_at(index, cap, L.i, 0);
+    return L;
+}
+template <int G>
+__device__ __forceinline__ float lane_sum(float v)
+{
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+constexpr int kDensG = 8, kViscG = 4;
+static unsigned list_blocks(int n, int lanes) { return (unsigned)(((long long)n * lanes + 255) / 256); }
+
+// 8 lanes per particle read the list's entries together; a thread per particle
+// took 47 us at 99k particles with a dynamic list, this 24.
 __global__ void __launch_bounds__(256)
     k_g_density(const float* __restrict__ x, int n, const int* __restrict__ index,
                 const int* __restrict__ elements, int cap, long long total, Spiky k, float mass,
                 float* __restrict__ rho, int* __restrict__ err)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float xi = x[3 * i], yi = x[3 * i + 1], zi = x[3 * i + 2], acc = 0.f;
-    int m = nb_size(index, cap, total, n, i);
-    for (int e = 0; e < m; ++e) {
-        int j = elements[nb_at(index, cap, i, e)];
+    const ListLane L = list_lane<kDensG>(index, cap, total, n);
+    const int i = L.i;
+    const float xi = x[3 * i], yi = x[3 * i + 1], zi = x[3 * i + 2];
+    float acc = 0.f;
+#pragma unroll 2
+    for (int e = L.sub; e < L.m; e += kDensG) {
+        const int j = elements[L.at + e];
         if (!valid_id(j, n, err)) continue;
-        float dx = xi - x[3 * j], dy = yi - x[3 * j + 1], dz = zi - x[3 * j + 2];
-        float r = sqrtf(dx * dx + dy * dy + dz * dz), w, g;
-        spiky_wg(k, r, w, g);
+        const float dx = xi - x[3 * j], dy = yi - x[3 * j + 1], dz = zi - x[3 * j + 2];
+        float w, g;
+        spiky_wg(k, sqrtf(dx * dx + dy * dy + dz * dz), w, g);
         acc += mass * w;
     }
-    rho[i] = acc;
+    acc = lane_sum<kDensG>(acc);
+    if (L.valid && L.sub == 0) rho[i] = acc;
 }
 
 __global__ void __launch_bounds__(256)
@@ -742,8 +859,7 @@ int density_generic(const float* x, int n, const int* index, const int* elements
                     long long total, const Spiky& k, float mass, float* rho, int* err, cudaStream_t st)
 {
     if (n <= 0) return 0;
-    k_g_density<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, n, index, elements, cap, total, k, mass, rho,
-                                                              err);
+    k_g_density<<<list_blocks(n, kDensG), 256, 0, st>>>(x, n, index, elements, cap, total, k, mass, rho, err);
     return 1;
 }
 
@@ -771,7 +887,7 @@ int pbd_generic_solve_scratch(float* x, float* v, int n, const int* index, const
     cudaMemcpyAsync(xold, x, sizeof(float) * (size_t)m3, cudaMemcpyDeviceToDevice, st);
     float* rho = rho_out != nullptr ? rho_out : rho_s;
     for (int it = 0; it < iterations; ++it) {
-        k_g_density<<<nb, 256, 0, st>>>(x, n, index, elements, cap, total, k, mass, rho, err);
+        k_g_density<<<list_blocks(n, kDensG), 256, 0, st>>>(x, n, index, elements, cap, total, k, mass, rho, err);
         k_g_lambda<<<nb, 256, 0, st>>>(x, rho, n, index, elements, cap, total, k, lam, dpos, err);
         k_g_disp<<<nb, 256, 0, st>>>(x, lam, n, index, elements, cap, total, k, dpos, err);
         k_g_add<<<nb3, 256, 0, st>>>(x, dpos, m3);
@@ -888,50 +1004,99 @@ SdfView sdf_view(const pk_ctx* c)
 }
 
 
-// ImplicitViscosity on any NeighborList<int> in caller order (one thread per
-// particle, as K_ApplyViscosity): vout from vin (the previous iterate) and vold.
+// ImplicitViscosity on any NeighborList<int> in caller order, 4 lanes per
+// particle on positions and velocities packed to 16 bytes.  The weights do not
+// change between the sweeps: where w is given, the first sweep keeps them in
+// the list's layout and their sums in vold's fourth value, and the others read
+// them (kMode 0: form, 1: form and keep, 2: read).  A thread per particle read a
+// sector for each entry and for each coordinate: 103 us a sweep at 262k
+// particles, now 60 after a first of 129 (which writes the weights).
+template <int kMode>
 __global__ void __launch_bounds__(256)
-    k_g_visc(const float* __restrict__ x, const float* __restrict__ vin, const float* __restrict__ vold,
-             float* __restrict__ vout, int n, const int* __restrict__ index, const int* __restrict__ elements,
-             int cap, long long total, ViscK k_, int* __restrict__ err)
+    k_g_visc(const float4* __restrict__ x, const float4* __restrict__ vin, float4* __restrict__ vold,
+             float4* __restrict__ vout, float* __restrict__ v_last, int n, const int* __restrict__ index,
+             const int* __restrict__ elements, int cap, long long total, ViscK k_, float* __restrict__ w_list,
+             int* __restrict__ err)
+{
+    const ListLane L = list_lane<kViscG>(index, cap, total, n);
+    const int i = L.i;
+    const float4 xi = __ldg(x + i);
+    float tw = 0.f, d0 = 0.f, d1 = 0.f, d2v = 0.f;
+#pragma unroll 4
+    for (int e = L.sub; e < L.m; e += kViscG) {
+        const int j = elements[L.at + e];
+        float w = 0.0f;
+        if (kMode == 2) w = __ldg(w_list + L.at + e);
+        if (!valid_id(j, n, err)) continue;
+        if (kMode != 2) {
+            const float4 xj = __ldg(x + j);
+            float d2, ir, dd;
+            pair_geom(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, k_.inv_h, d2, ir, dd);
+            w = d2 > kEps2 ? k_.cw * dd : 0.0f;
+            if (kMode == 1) w_list[L.at + e] = w;
+            tw += w;
+        }
+        const float4 vj = __ldg(vin + j);
+        d0 = fmaf(w, vj.x, d0);
+        d1 = fmaf(w, vj.y, d1);
+        d2v = fmaf(w, vj.z, d2v);
+    }
+    d0 = lane_sum<kViscG>(d0);
+    d1 = lane_sum<kViscG>(d1);
+    d2v = lane_sum<kViscG>(d2v);
+    if (kMode != 2) tw = lane_sum<kViscG>(tw);
+    if (!L.valid || L.sub != 0) return;
+    const float4 vo = vold[i];
+    if (kMode == 2) tw = vo.w;
+    if (kMode == 1) vold[i].w = tw;
+    const float b = tw < kEpsilon ? 0.0f : k_.b;
+    const float t = tw < kEpsilon ? 1.0f : tw;
+    const float4 r = visc_mix(vo, d0, d1, d2v, b, t);
+    if (v_last != nullptr) {
+        v_last[3LL * i] = r.x;
+        v_last[3LL * i + 1] = r.y;
+        v_last[3LL * i + 2] = r.z;
+    } else {
+        vout[i] = r;
+    }
+}
+
+__global__ void __launch_bounds__(256)
+    k_g_pack(const float* __restrict__ x, const float* __restrict__ v, int n, float4* __restrict__ x4,
+             float4* __restrict__ v4, float4* __restrict__ vold)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float xi0 = x[3 * i], xi1 = x[3 * i + 1], xi2 = x[3 * i + 2];
-    float tw = 0.f, d0 = 0.f, d1 = 0.f, d2v = 0.f;
-    const int m = nb_size(index, cap, total, n, i);
-    for (int e = 0; e < m; ++e) {
-        const int j = elements[nb_at(index, cap, i, e)];
-        if (!valid_id(j, n, err)) continue;
-        float d2, ir, dd;
-        pair_geom(xi0 - x[3 * j], xi1 - x[3 * j + 1], xi2 - x[3 * j + 2], k_.inv_h, d2, ir, dd);
-        const float w = d2 > kEps2 ? k_.cw * dd : 0.0f;
-        tw += w;
-        d0 = fmaf(w, vin[3 * j], d0);
-        d1 = fmaf(w, vin[3 * j + 1], d1);
-        d2v = fmaf(w, vin[3 * j + 2], d2v);
-    }
-    const float b = tw < kEpsilon ? 0.0f : k_.b;
-    const float t = tw < kEpsilon ? 1.0f : tw;
-    vout[3 * i] = vold[3 * i] / (1.0f + b) + d0 / t * b / (1.0f + b);
-    vout[3 * i + 1] = vold[3 * i + 1] / (1.0f + b) + d1 / t * b / (1.0f + b);
-    vout[3 * i + 2] = vold[3 * i + 2] / (1.0f + b) + d2v / t * b / (1.0f + b);
+    const long long o = 3LL * i;
+    x4[i] = make_float4(x[o], x[o + 1], x[o + 2], 0.f);
+    const float4 u = make_float4(v[o], v[o + 1], v[o + 2], 0.f);
+    v4[i] = u;
+    vold[i] = u;
 }
 
 int viscosity_generic(pk_ctx* c, const float* x, float* v, int n, const int* index, const int* elements, int cap,
                       long long total, float vis, float h, int iterations, float dt, cudaStream_t st)
 {
     if (n <= 0 || iterations <= 0) return 0;
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    const size_t bytes = sizeof(float) * 3 * (size_t)n;
     const ViscK vk = visc_k(vis, h, dt);
-    // velOld and velBuf copies, then the sweep (ImplicitViscosity.cu:105-124)
-    cudaMemcpyAsync(c->g_xold, v, bytes, cudaMemcpyDeviceToDevice, st);
+    float4 *x4 = c->g_quads, *vold = x4 + n, *va = vold + n, *vb = va + n;
+    // no room for the weights, or a single sweep: every sweep forms them
+    float* const w = iterations > 1 && c->g_w_cap >= (cap > 0 ? (long long)n * cap : total) ? c->g_w : nullptr;
+    k_g_pack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, v, n, x4, va, vold);
     for (int t = 0; t < iterations; ++t) {
-        cudaMemcpyAsync(c->g_dpos, v, bytes, cudaMemcpyDeviceToDevice, st);
-        k_g_visc<<<nb, 256, 0, st>>>(x, c->g_dpos, c->g_xold, v, n, index, elements, cap, total, vk, c->d_err);
+        float* const last = t == iterations - 1 ? v : nullptr;
+        if (w == nullptr)
+            k_g_visc<0><<<list_blocks(n, kViscG), 256, 0, st>>>(x4, va, vold, vb, last, n, index, elements, cap, total, vk, w,
+                                                        c->d_err);
+        else if (t == 0)
+            k_g_visc<1><<<list_blocks(n, kViscG), 256, 0, st>>>(x4, va, vold, vb, last, n, index, elements, cap, total, vk, w,
+                                                        c->d_err);
+        else
+            k_g_visc<2><<<list_blocks(n, kViscG), 256, 0, st>>>(x4, va, vold, vb, last, n, index, elements, cap, total, vk, w,
+                                                        c->d_err);
+        std::swap(va, vb);
     }
-    return iterations;
+    return 1 + iterations;
 }
 
 }  // namespace pk

@@ -62,7 +62,7 @@ def test_builds_on_one_context_equal_fresh_ones():
     one.close()
 
 
-@pytest.mark.parametrize("viscosity", [0.0])
+@pytest.mark.parametrize("viscosity", [0.0, 1.0])
 def test_row_walks_of_small_and_large_scenes_agree(viscosity):
     # each scene alone keeps several quads per thread in flight, both together
     # (77,788 particles) one: the same sums in the same order
@@ -84,6 +84,21 @@ def test_row_walks_of_small_and_large_scenes_agree(viscosity):
         assert torch.equal(x, xb[off[k]:off[k + 1]]) and torch.equal(v, vb[off[k]:off[k + 1]])
     ctx.check_status()
     ctx.close()
+
+
+@pytest.mark.parametrize("cap", [37, 0])
+@pytest.mark.parametrize("iterations", [1, 2])
+def test_viscosity_sweeps_on_a_list(ctx, oracle, cap, iterations):
+    # the first sweep forms the weights, the later ones read them
+    sc = scenes.dam_break_small(seed=17, n_side=11)
+    v0 = np.random.default_rng(17).normal(0, 0.3, sc.x.shape).astype(np.float32)
+    ri, re = oracle.neighbor_query(sc.x, sc.radius, sc.lo, sc.hi, cap)
+    total = re.shape[0] if cap == 0 else sc.x.shape[0] * cap
+    v = t(v0)
+    ctx.viscosity(t(sc.x), v, t(ri, np.int32), t(re, np.int32), cap, total, 1.0, sc.radius, iterations, sc.dt)
+    ctx.check_status()
+    vo = oracle.implicit_viscosity(sc.x, v0, ri, re, cap, 1.0, sc.radius, iterations, sc.dt)
+    assert rel(v.cpu().numpy(), vo) < 1e-5
 
 
 def bar(ctx, oracle, ratio, cap, seed=0):
