@@ -182,43 +182,108 @@ __global__ void __launch_bounds__(256)
     vb[3 * i + 2] += dt * y0z;
 }
 
-// r1: at iterate y_t, lambda_i, rhobar_i, Dbar_i (q1) and S_i (q2).
-template <class T>
-__global__ void __launch_bounds__(kAdjBlock, 4)
-    k_adj_r1(const T* __restrict__ y, const double4* __restrict__ a, const int* __restrict__ rows,
-             const int2* __restrict__ rcnt, int row_cap, int n, AdjK K, double4* __restrict__ q1,
-             double4* __restrict__ q2)
+// What r2 gathers of a neighbour besides y and a: 48 bytes in three 16-byte
+// loads.
+struct alignas(16) AdjQ {
+    double lam, rb, Db, Sx, Sy, Sz;
+};
+__device__ __forceinline__ AdjQ ldq(const AdjQ* p)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const double3 yi = ld3(y, s);
-    const double4 ai4 = a[s];
-    const double3 ai = make_double3(ai4.x, ai4.y, ai4.z);
-    const int nu = rcnt[s].y;
+    const double2* d = reinterpret_cast<const double2*>(p);
+    const double2 a = __ldg(d), b = __ldg(d + 1), c = __ldg(d + 2);
+    return AdjQ{a.x, a.y, b.x, b.y, c.x, c.y};
+}
+__device__ __forceinline__ double3 ld3d(const double4* p, int s)
+{
+    const double2* d = reinterpret_cast<const double2*>(p + s);
+    const double2 a = __ldg(d);
+    return make_double3(a.x, a.y, __ldg(reinterpret_cast<const double*>(d + 1)));
+}
+
+// Both reverse kernels run kRevG lanes per particle, lane `sub` taking row
+// quads sub, sub + kRevG, ... (8 particles' quads are 128 contiguous bytes), so
+// a block of 65,536 particles fills the chip; sums are combined with xor
+// shuffles in a fixed order.  1/r comes from one double reciprocal square root
+// (r = r2/sqrt(r2)): no square root or division per entry.
+constexpr int kRevG = 4;
+__device__ __forceinline__ double rsum(double v)
+{
+#pragma unroll
+    for (int o = kRevG / 2; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+struct RevLane {
+    int s, sub, m;
+    bool valid;
+    const int4* rq;
+};
+__device__ __forceinline__ RevLane rev_lane(const int* rows, const int2* rcnt, int row_cap, int n)
+{
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    RevLane L;
+    L.s = gid / kRevG;
+    L.sub = gid % kRevG;
+    L.valid = L.s < n;
+    if (!L.valid) L.s = n - 1;
+    L.m = rcnt[L.s].y;
+    L.rq = reinterpret_cast<const int4*>(rows + row_slot(L.s, 0, row_cap));
+    return L;
+}
+// Calls f on every row entry of the lane's quads.
+template <class F>
+__device__ __forceinline__ void rev_walk(const RevLane& L, const F& f)
+{
+    const int nq = (L.m + 3) >> 2;
+    int4 nxt = L.sub < nq ? __ldg(L.rq + 32LL * L.sub) : make_int4(0, 0, 0, 0);
+    for (int q = L.sub; q < nq; q += kRevG) {
+        const int4 cur = nxt;
+        if (q + kRevG < nq) nxt = __ldg(L.rq + 32LL * (q + kRevG));
+        const int ent[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (4 * q + k < L.m) f(ent[k]);
+    }
+}
+
+// r1: at iterate y_t, lambda_i, rhobar_i, Dbar_i and S_i.  The kernel's
+// constants multiply the finished sums.  Both passes are bound by double
+// arithmetic: kRevG lanes per particle and one reciprocal square root in place
+// of a square root and a division take 28 and 48 us at 65k particles, a thread
+// per particle with both took 53 and 67.
+template <class T>
+__global__ void __launch_bounds__(kAdjBlock)
+    k_adj_r1(const T* __restrict__ y, const double4* __restrict__ a, const int* __restrict__ rows,
+             const int2* __restrict__ rcnt, int row_cap, int n, AdjK K, AdjQ* __restrict__ out)
+{
+    const RevLane L = rev_lane(rows, rcnt, row_cap, n);
+    const double3 yi = ld3(y, L.s), ai = ld3d(a, L.s);
     double rho = 0.0, sg = 0.0, lb = 0.0;
     double3 S = make_double3(0.0, 0.0, 0.0);
-    for (int e = 0; e < nu; ++e) {
-        const int v = rows[row_slot(s, e, row_cap)];
+    rev_walk(L, [&](int v) {
         const int j = v & kRowIndexMask;
-        const bool A = v < 0;  // bit 31: j in N(i)
-        const double mult = (double)__popc((unsigned)v >> 30);
-        const double3 d = sub3(yi, ld3(y, j));
-        const double r2 = dot3(d, d), r = sqrt(r2);
-        const double om = fmax(1.0 - r * K.inv_h, 0.0);
-        if (A) rho += K.m * K.cw * om * om * om;
+        const double3 yj = ld3(y, j), aj = ld3d(a, j);
+        const double wa = v < 0 ? 1.0 : 0.0;  // bit 31: j in N(i)
+        const double mult = (unsigned)v >= 0xc0000000u ? 2.0 : 1.0;
+        const double3 d = sub3(yi, yj);
+        const double r2 = dot3(d, d), ir = rsqrt(fmax(r2, 1e-60));
+        const double om = fmax(fma(-(r2 * ir), K.inv_h, 1.0), 0.0), om2 = om * om;
+        rho += wa * om2 * om;
         if (r2 > kAdjEps2) {
-            const double w1 = K.cg * om * om, c = w1 / r;
-            const double3 P = make_double3(c * d.x, c * d.y, c * d.z);
-            if (A) {
-                S.x += P.x;
-                S.y += P.y;
-                S.z += P.z;
-                sg += w1 * w1;
-            }
-            const double4 aj = a[j];
-            lb += mult * (P.x * (ai.x - aj.x) + P.y * (ai.y - aj.y) + P.z * (ai.z - aj.z));
+            const double c = om2 * ir, ca = wa * c;
+            S.x += ca * d.x;
+            S.y += ca * d.y;
+            S.z += ca * d.z;
+            sg += wa * (om2 * om2);
+            lb += mult * c * (d.x * (ai.x - aj.x) + d.y * (ai.y - aj.y) + d.z * (ai.z - aj.z));
         }
-    }
+    });
+    rho = K.m * K.cw * rsum(rho);
+    sg = K.cg * K.cg * rsum(sg);
+    lb = K.cg * rsum(lb);
+    S.x = K.cg * rsum(S.x);
+    S.y = K.cg * rsum(S.y);
+    S.z = K.cg * rsum(S.z);
+    if (!L.valid || L.sub != 0) return;
     const double D = sg + dot3(S, S) + 0.1;
     const double lraw = -(rho - 1000.0) / D;
     const double lam = lraw > 0.0 ? 0.0 : lraw;
@@ -228,49 +293,59 @@ __global__ void __launch_bounds__(kAdjBlock, 4)
         rb = -lbar / D;
         Db = -lbar * lam / D;
     }
-    q1[s] = make_double4(lam, rb, Db, 0.0);
-    q2[s] = make_double4(S.x, S.y, S.z, 0.0);
+    double2* const o = reinterpret_cast<double2*>(out + L.s);
+    o[0] = make_double2(lam, rb);
+    o[1] = make_double2(Db, S.x);
+    o[2] = make_double2(S.y, S.z);
 }
 
-// r2: dL/dy_t.
+// r2: dL/dy_t.  With P = w1 u and f = w1/r, an entry's term
+// J vec + cr P = w2 u (u.vec) + f (vec - u (u.vec)) + cr P is
+// f vec + u ((w2 - f) u.vec + cr w1).
 template <class T>
-__global__ void __launch_bounds__(kAdjBlock, 4)
-    k_adj_r2(const T* __restrict__ y, const double4* __restrict__ a, const double4* __restrict__ q1,
-             const double4* __restrict__ q2, const int* __restrict__ rows, const int2* __restrict__ rcnt,
-             int row_cap, int n, AdjK K, double4* __restrict__ out)
+__global__ void __launch_bounds__(kAdjBlock)
+    k_adj_r2(const T* __restrict__ y, const double4* __restrict__ a, const AdjQ* __restrict__ qs,
+             const int* __restrict__ rows, const int2* __restrict__ rcnt, int row_cap, int n, AdjK K,
+             double4* __restrict__ out)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const double3 yi = ld3(y, s);
-    const double4 ai = a[s], qi = q1[s], Si = q2[s];
-    const int nu = rcnt[s].y;
-    double ox = ai.x, oy = ai.y, oz = ai.z;
-    for (int e = 0; e < nu; ++e) {
-        const int v = rows[row_slot(s, e, row_cap)];
+    const RevLane L = rev_lane(rows, rcnt, row_cap, n);
+    const double3 yi = ld3(y, L.s), ai = ld3d(a, L.s);
+    const AdjQ qi = ldq(qs + L.s);
+    const double minv = K.m * K.inv_h;  // dW/dr = G/h
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+    rev_walk(L, [&](int v) {
         const int j = v & kRowIndexMask;
-        const double3 d = sub3(yi, ld3(y, j));
+        const double3 yj = ld3(y, j), aj = ld3d(a, j);
+        const AdjQ qj = ldq(qs + j);
+        const double3 d = sub3(yi, yj);
         const double r2 = dot3(d, d);
-        if (!(r2 > kAdjEps2)) continue;
-        const double A = v < 0 ? 1.0 : 0.0, B = ((v >> 30) & 1) ? 1.0 : 0.0;
-        const double r = sqrt(r2), ir = 1.0 / r;
+        if (!(r2 > kAdjEps2)) return;
+        const bool A = v < 0, B = ((v >> 30) & 1) != 0;
+        const double ir = rsqrt(r2);
         const double3 u = make_double3(d.x * ir, d.y * ir, d.z * ir);
-        const double om = fmax(1.0 - r * K.inv_h, 0.0);
+        const double om = fmax(fma(-(r2 * ir), K.inv_h, 1.0), 0.0);
         const double w1 = K.cg * om * om, w2 = -2.0 * K.cg * om * K.inv_h;
-        const double3 P = make_double3(w1 * u.x, w1 * u.y, w1 * u.z);
-        const double4 aj = a[j], qj = q1[j], Sj = q2[j];
-        const double cl = 10.0 * (A + B) * (qi.x + qj.x);
-        const double ca = 2.0 * A * qi.z, cb = 2.0 * B * qj.z;
-        const double3 vec = make_double3(cl * (ai.x - aj.x) + ca * (P.x + Si.x) + cb * (P.x - Sj.x),
-                                         cl * (ai.y - aj.y) + ca * (P.y + Si.y) + cb * (P.y - Sj.y),
-                                         cl * (ai.z - aj.z) + ca * (P.z + Si.z) + cb * (P.z - Sj.z));
-        const double uv = dot3(u, vec);
+        const double cl = (A && B ? 20.0 : 10.0) * (qi.lam + qj.lam);
+        const double ca = A ? 2.0 * qi.Db : 0.0, cb = B ? 2.0 * qj.Db : 0.0;
+        const double cab = (ca + cb) * w1;
+        const double3 vec = make_double3(cl * (ai.x - aj.x) + cab * u.x + (ca * qi.Sx - cb * qj.Sx),
+                                         cl * (ai.y - aj.y) + cab * u.y + (ca * qi.Sy - cb * qj.Sy),
+                                         cl * (ai.z - aj.z) + cab * u.z + (ca * qi.Sz - cb * qj.Sz));
         const double f = w1 * ir;
-        const double cr = K.m * K.inv_h * (A * qi.y + B * qj.y);  // dW/dr = G/h
-        ox += w2 * u.x * uv + f * (vec.x - u.x * uv) + cr * P.x;
-        oy += w2 * u.y * uv + f * (vec.y - u.y * uv) + cr * P.y;
-        oz += w2 * u.z * uv + f * (vec.z - u.z * uv) + cr * P.z;
+        const double cr = minv * ((A ? qi.rb : 0.0) + (B ? qj.rb : 0.0));
+        const double g = (w2 - f) * dot3(u, vec) + cr * w1;
+        ox += f * vec.x + g * u.x;
+        oy += f * vec.y + g * u.y;
+        oz += f * vec.z + g * u.z;
+    });
+    ox = rsum(ox);
+    oy = rsum(oy);
+    oz = rsum(oz);
+    if (L.valid && L.sub == 0) {
+        double2* const o = reinterpret_cast<double2*>(out + L.s);
+        o[0] = make_double2(ai.x + ox, ai.y + oy);
+        o[1] = make_double2(ai.z + oz, 0.0);
     }
-    out[s] = make_double4(ox, oy, oz, 0.0);
 }
 
 __global__ void __launch_bounds__(256) k_to_double(const float* __restrict__ a, long long m, double* __restrict__ b)
@@ -317,7 +392,8 @@ struct PbdRoll {
     double4 *y64a = nullptr, *y64b = nullptr, *y64c = nullptr, *vp64 = nullptr;
     double* lam64 = nullptr;
     // reverse state
-    double4 *a = nullptr, *a2 = nullptr, *q1 = nullptr, *q2 = nullptr;
+    double4 *a = nullptr, *a2 = nullptr;
+    AdjQ* q = nullptr;
     double *xb = nullptr, *vb = nullptr;
     // replay state (caller order) of the double and of the float rollout
     double *xw64 = nullptr, *vw64 = nullptr;
@@ -353,7 +429,7 @@ bool ensure_roll_n(PbdRoll& R, int n)
     const size_t m = (size_t)n;
     const bool ok = realloc_to(R.xf, 3 * m) && realloc_to(R.y64a, m) && realloc_to(R.y64b, m) &&
                     realloc_to(R.y64c, m) && realloc_to(R.vp64, m) && realloc_to(R.lam64, m) &&
-                    realloc_to(R.a, m) && realloc_to(R.a2, m) && realloc_to(R.q1, m) && realloc_to(R.q2, m) &&
+                    realloc_to(R.a, m) && realloc_to(R.a2, m) && realloc_to(R.q, m) &&
                     realloc_to(R.xb, 3 * m) && realloc_to(R.vb, 3 * m) && realloc_to(R.xw64, 3 * m) &&
                     realloc_to(R.vw64, 3 * m) && realloc_to(R.xw32, 3 * m) && realloc_to(R.vw32, 3 * m);
     if (!ok) return false;
@@ -480,7 +556,7 @@ int reverse_segment(PbdRoll& R, const T* ys_base, int len, cudaStream_t st)
     const long long slots = row_slots(n, R.row_cap);
     const AdjK K = adj_k(R);
     const double dt = (double)R.dt, inv_dt = 1.0 / dt;
-    const unsigned nb = blocks_of(n, kAdjBlock), nb256 = blocks_of(n, 256);
+    const unsigned nb = blocks_of((long long)n * kRevG, kAdjBlock), nb256 = blocks_of(n, 256);
     int l = 0;
     for (int j = len - 1; j >= 0; --j) {
         const int* perm = R.seg_perm + (size_t)j * n;
@@ -490,8 +566,8 @@ int reverse_segment(PbdRoll& R, const T* ys_base, int len, cudaStream_t st)
         k_adj_init<<<nb256, 256, 0, st>>>(perm, n, R.xb, R.vb, inv_dt, R.a);
         for (int it = R.iterations - 1; it >= 0; --it) {
             const T* y = ys + (size_t)it * n;
-            k_adj_r1<T><<<nb, kAdjBlock, 0, st>>>(y, R.a, rows, rcnt, R.row_cap, n, K, R.q1, R.q2);
-            k_adj_r2<T><<<nb, kAdjBlock, 0, st>>>(y, R.a, R.q1, R.q2, rows, rcnt, R.row_cap, n, K, R.a2);
+            k_adj_r1<T><<<nb, kAdjBlock, 0, st>>>(y, R.a, rows, rcnt, R.row_cap, n, K, R.q);
+            k_adj_r2<T><<<nb, kAdjBlock, 0, st>>>(y, R.a, R.q, rows, rcnt, R.row_cap, n, K, R.a2);
             std::swap(R.a, R.a2);
         }
         k_adj_final<<<nb256, 256, 0, st>>>(perm, n, R.a, dt, inv_dt, R.xb, R.vb);
@@ -521,7 +597,7 @@ void pbd_roll_release(pk_ctx* c)
     PbdRoll* R = roll_of(c);
     if (!R) return;
     void* ps[] = {R->ck32, R->ck64, R->seg_perm, R->seg_rows, R->seg_rcnt, R->seg_y32, R->seg_y64, R->xf,
-                  R->y64a, R->y64b, R->y64c, R->vp64, R->lam64, R->a, R->a2, R->q1, R->q2, R->xb, R->vb,
+                  R->y64a, R->y64b, R->y64c, R->vp64, R->lam64, R->a, R->a2, R->q, R->xb, R->vb,
                   R->xw64, R->vw64, R->xw32, R->vw32};
     for (void* p : ps)
         if (p) cudaFree(p);
