@@ -1379,8 +1379,9 @@ PK_API int pk_pd_rotate_rest_shape(pk_ctx* c, const float* x, int n, float horiz
     if (n > 0 && !x) return fail(c, PK_ERR_ARG, "null positions");
     cudaSetDevice(c->device);
     if ((rc = ensure_plastic(c))) return rc;
-    ++c->pd_shape_rev;
     c->launches = pk::pl_rotate(c, x, horizon, (cudaStream_t)stream);
+    ++c->pd_shape_rev;
+    if (c->launches < 0) return fail(c, PK_ERR_NOMEM, "device allocation of the projection workspace failed");
     return check_launch(c, "pk_pd_rotate_rest_shape");
 }
 
@@ -1391,8 +1392,9 @@ PK_API int pk_pd_apply_yielding(pk_ctx* c, const float* x, int n, const pk_plast
     if (rc) return rc;
     cudaSetDevice(c->device);
     if ((rc = ensure_plastic(c))) return rc;
-    ++c->pd_shape_rev;
     c->launches = pk::pl_yield(c, x, p, (cudaStream_t)stream);
+    ++c->pd_shape_rev;
+    if (c->launches < 0) return fail(c, PK_ERR_NOMEM, "device allocation of the projection workspace failed");
     return check_launch(c, "pk_pd_apply_yielding");
 }
 
@@ -1403,6 +1405,7 @@ PK_API int pk_pd_fracture(pk_ctx* c, const float* x, int n, const pk_plastic_par
     if (rc) return rc;
     cudaSetDevice(c->device);
     c->launches = pk::pl_fracture(c, x, p, (cudaStream_t)stream);
+    if (c->launches < 0) return fail(c, PK_ERR_NOMEM, "device allocation of the projection workspace failed");
     return check_launch(c, "pk_pd_fracture");
 }
 

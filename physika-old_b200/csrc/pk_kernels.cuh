@@ -63,6 +63,7 @@ int pd_inverse_k(pk_ctx* c, float horizon, cudaStream_t st);
 int pd_begin(pk_ctx* c, const float* x, int n, float horizon, float mu, float lambda, cudaStream_t st);
 int pd_enforce(pk_ctx* c, float* x, int n, float horizon, float mu, float lambda, cudaStream_t st);
 int pd_update_velocity(pk_ctx* c, const float* x, float* v, int n, float dt, cudaStream_t st);
+const float4* pd_pack(pk_ctx* c, const float* x, bool bonds, int& launches, cudaStream_t st);
 // pk_plastic.cu
 constexpr int kPlMk = 20;  // floats per particle of the rotation scratch (pk_ctx::pl_mk)
 int pl_rotate(pk_ctx* c, const float* x, float h, cudaStream_t st);

@@ -1091,6 +1091,20 @@ int pd_project_solve(pk_ctx* c, float* x, float* v, int n, float horizon, float 
     return l + 1 + project<float>(*w, B, x, v, c->pd_bulk, iterations, dt, stretch, st);
 }
 
+// The caller's positions packed to 16 bytes (in scratch the next projection
+// overwrites), with the compact bonds brought up to date where they are asked
+// for; null when memory runs out.
+const float4* pd_pack(pk_ctx* c, const float* x, bool bonds, int& launches, cudaStream_t st)
+{
+    const int n = c->pd_n;
+    PdWork<float>*& w = work_of<float>(c);
+    if (!w) w = new PdWork<float>();
+    if (bonds ? !ensure_work<float>(c, n, st, launches) : !work_alloc(*w, n)) return nullptr;
+    k_pd_pack<float><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, x, w->xa);
+    ++launches;
+    return reinterpret_cast<const float4*>(w->xa);
+}
+
 // The projection one step at a time (pk_pd_begin / pk_pd_enforce /
 // pk_pd_update_velocity): x_old is kept in the float workspace between the
 // calls (the bond weights come with every iteration's bond terms).

@@ -24,6 +24,40 @@ struct RestView {
     const int* ridx;
     float* rpos;
 };
+// The same shape as the projection's compact bonds (pk_pd_adj.cu): rest_j -
+// rest_i and j (~j for a broken bond, which plasticity moves like any other) in
+// one 16-byte load, in ascending order of j; positions packed to 16 bytes.  The
+// rotation's sums walk these (82 -> 56 us at 65,536 particles with 113 bonds).
+// The kernels after it read and write the rest shape in its own order: writing
+// it bond by bond in the compact order took 235-250 us (partly written sectors)
+// against 38 and 70.
+struct BondView {
+    const float4* bond;
+    const float4* x;
+};
+// Bonds a lane has in flight.
+constexpr int kPlU = 4;
+__device__ __forceinline__ int bond_j(const float4& b)
+{
+    const int j = __float_as_int(b.w);
+    return j >= 0 ? j : ~j;
+}
+// Calls f(place in the row, bond, x_j) on the lane's bonds, in order.
+template <class F>
+__device__ __forceinline__ void walk_bonds(const BondView& V, long long a0, int m, int sub, int i, const F& f)
+{
+    for (int e0 = sub; e0 < m; e0 += 8 * kPlU) {
+        float4 b[kPlU], xj[kPlU];
+#pragma unroll
+        for (int u = 0; u < kPlU; ++u)
+            b[u] = e0 + 8 * u < m ? V.bond[a0 + e0 + 8 * u] : make_float4(0.f, 0.f, 0.f, __int_as_float(i));
+#pragma unroll
+        for (int u = 0; u < kPlU; ++u) xj[u] = __ldg(V.x + bond_j(b[u]));
+#pragma unroll
+        for (int u = 0; u < kPlU; ++u)
+            if (e0 + 8 * u < m) f(e0 + 8 * u, b[u], xj[u]);
+    }
+}
 
 __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf((x * x + y * y) + z * z); }
 
@@ -171,27 +205,20 @@ __device__ inline float det3f(const float M[3][3])
 // rotation (two double-precision eigen-decompositions, every lane of a warp
 // busy with its own particle), and kPlG lanes per particle rotate the bonds.
 // Scratch per particle (kPlMk floats): mat (9), K (9), tw; then R (9).
-__global__ void __launch_bounds__(kPlBlock) k_pl_rot_sums(RestView R, const float* __restrict__ x, float h,
-                                                          float* __restrict__ mk)
+__global__ void __launch_bounds__(kPlBlock) k_pl_rot_sums(RestView R, BondView V, float h, float* __restrict__ mk)
 {
     const PlLane L = pl_lane(R.n);
     const int i = L.i;
     const long long a0 = pd_at(R.index, R.cap, i, 0);
-    const float ri[3] = {R.rpos[3 * a0], R.rpos[3 * a0 + 1], R.rpos[3 * a0 + 2]};
     const int m = pd_size(R.index, R.cap, R.total, R.n, i);
+    const float4 xi = __ldg(V.x + i);
     float tw = 0.f, mat[3][3] = {}, K[3][3] = {};
-    for (int e = L.sub; e < m; e += kPlG) {
-        const long long at = pd_at(R.index, R.cap, i, e);
-        const int j = R.ridx[at];
-        const float* rj = R.rpos + 3 * at;
-        const float r = len3(ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]);
+    walk_bonds(V, a0, m, L.sub, i, [&](int, const float4& d, const float4& xj) {
+        const float r = len3(d.x, d.y, d.z);
         if (r > kEpsilon) {
             const float wt = smooth_w(r, h);
-            float p[3], q[3];
-            for (int a = 0; a < 3; ++a) {
-                p[a] = (x[3 * j + a] - x[3 * i + a]) / h;
-                q[a] = (rj[a] - ri[a]) / h;
-            }
+            const float p[3] = {(xj.x - xi.x) / h, (xj.y - xi.y) / h, (xj.z - xi.z) / h};
+            const float q[3] = {d.x / h, d.y / h, d.z / h};
             for (int a = 0; a < 3; ++a)
                 for (int b = 0; b < 3; ++b) {
                     mat[a][b] += p[a] * q[b] * wt;
@@ -199,7 +226,7 @@ __global__ void __launch_bounds__(kPlBlock) k_pl_rot_sums(RestView R, const floa
                 }
             tw += wt;
         }
-    }
+    });
     gsum8(mat);
     gsum8(K);
     tw = gsum8(tw);
@@ -264,54 +291,64 @@ __global__ void __launch_bounds__(kPlBlock) k_pl_rot_apply(RestView R, const flo
 }
 
 // I1 and the reference's J2 (PM_ComputeInvariants, ElastoplasticityModule.cu:43-128;
-// the J2 loop assigns, so only the last bond over 0.01 h counts), by the
-// particle's lane group: the I1 sums are combined, and J2 is the term of the
-// group's largest qualifying bond index.
-__device__ inline void invariants(const RestView& R, const float* __restrict__ x, float h, int i, int sub,
-                                  float& I1, float& J2)
+// the J2 loop assigns, so only the last bond over 0.01 h of the list counts),
+// by the particle's lane group on the packed positions x, kPlU bonds in flight:
+// the I1 sums are combined, and J2 is the term of the last qualifying bond,
+// looked for from the end of the row.
+__device__ inline void invariants(const RestView& R, const float4* __restrict__ x, float h, int i, int sub, float& I1,
+                                  float& J2)
 {
     const long long a0 = pd_at(R.index, R.cap, i, 0);
     const float ri[3] = {R.rpos[3 * a0], R.rpos[3 * a0 + 1], R.rpos[3 * a0 + 2]};
     const int m = pd_size(R.index, R.cap, R.total, R.n, i);
+    const float4 xi = __ldg(x + i);
     const double lim = 0.01 * (double)h;
+    auto length = [&](float4 xj) { return len3(xj.x - xi.x, xj.y - xi.y, xj.z - xi.z); };
     float s1 = 0.f, tw = 0.f;
-    for (int e = 1 + sub; e < m; e += kPlG) {
-        const long long at = pd_at(R.index, R.cap, i, e);
-        const int j = R.ridx[at];
-        const float* rj = R.rpos + 3 * at;
-        const float r = len3(ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]);
-        if ((double)r > lim) {
-            const float wt = corr_w(r, h);
-            const float pl = len3(x[3 * j] - x[3 * i], x[3 * j + 1] - x[3 * i + 1], x[3 * j + 2] - x[3 * i + 2]);
-            s1 += wt * (pl / r);
-            tw += wt;
+    for (int e0 = 1 + sub; e0 < m; e0 += kPlG * kPlU) {
+        float r[kPlU];
+        float4 xj[kPlU];
+#pragma unroll
+        for (int u = 0; u < kPlU; ++u) {
+            const int e = e0 + u * kPlG;
+            const bool in = e < m;
+            const float* rj = R.rpos + 3 * (in ? a0 + e : a0);
+            r[u] = in ? len3(ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]) : 0.f;
+            xj[u] = __ldg(x + (in ? R.ridx[a0 + e] : i));
         }
+#pragma unroll
+        for (int u = 0; u < kPlU; ++u)
+            if ((double)r[u] > lim) {
+                const float wt = corr_w(r[u], h);
+                s1 += wt * (length(xj[u]) / r[u]);
+                tw += wt;
+            }
     }
     s1 = gsum8(s1);
     tw = gsum8(tw);
     s1 = tw > kEpsilon ? s1 / tw : 1.0f;
     int last = -1;
     float j2 = 0.f;
-    for (int e = 1 + sub; e < m; e += kPlG) {
-        const long long at = pd_at(R.index, R.cap, i, e);
-        const int j = R.ridx[at];
-        const float* rj = R.rpos + 3 * at;
-        const float r = len3(ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]);
-        if ((double)r > lim) {
-            const float wt = corr_w(r, h);
-            const float pl = len3(x[3 * j] - x[3 * i], x[3 * j + 1] - x[3 * i + 1], x[3 * j + 2] - x[3 * i + 2]);
-            const float ratio = pl / r;
-            j2 = (ratio - s1) * (ratio - s1) * wt;
-            last = e;
+    for (int top = m - 1; __any_sync(0xffffffffu, last < 0 && top >= 1); top -= kPlG) {
+        const int e = top - sub;
+        if (last < 0 && e >= 1) {
+            const long long at = a0 + e;
+            const float* rj = R.rpos + 3 * at;
+            const float r = len3(ri[0] - rj[0], ri[1] - rj[1], ri[2] - rj[2]);
+            if ((double)r > lim) {
+                const float ratio = length(__ldg(x + R.ridx[at])) / r;
+                j2 = (ratio - s1) * (ratio - s1) * corr_w(r, h);
+                last = e;
+            }
         }
-    }
 #pragma unroll
-    for (int o = kPlG / 2; o >= 1; o >>= 1) {
-        const int ol = __shfl_xor_sync(0xffffffffu, last, o);
-        const float oj = __shfl_xor_sync(0xffffffffu, j2, o);
-        if (ol > last) {
-            last = ol;
-            j2 = oj;
+        for (int o = kPlG / 2; o >= 1; o >>= 1) {
+            const int ol = __shfl_xor_sync(0xffffffffu, last, o);
+            const float oj = __shfl_xor_sync(0xffffffffu, j2, o);
+            if (ol > last) {
+                last = ol;
+                j2 = oj;
+            }
         }
     }
     I1 = s1;
@@ -320,9 +357,9 @@ __device__ inline void invariants(const RestView& R, const float* __restrict__ x
 
 // PM_ComputeInvariants: Drucker-Prager yield (a yielding particle keeps its flag).
 __global__ void __launch_bounds__(kPlBlock)
-    k_pl_invariants(RestView R, const float* __restrict__ x, const float* __restrict__ bulk, float h, float A,
-                    float B, float mu, float lambda, float* __restrict__ y1, float* __restrict__ y2,
-                    float* __restrict__ i1, unsigned char* __restrict__ byield)
+    k_pl_invariants(RestView R, const float4* __restrict__ x, const float* __restrict__ bulk, float h, float A,
+                    float B, float mu, float lambda, float* __restrict__ y1, float* __restrict__ y2, float* __restrict__ i1,
+                    unsigned char* __restrict__ byield, float4* __restrict__ y4)
 {
     const PlLane L = pl_lane(R.n);
     const int i = L.i;
@@ -332,18 +369,19 @@ __global__ void __launch_bounds__(kPlBlock)
     const float sJ2 = J2 * mu * bulk[i];
     const float sD1 = (1.0f - I1) * lambda * bulk[i];
     const float lim = A + B * sD1;
+    float a = 0.f, b = 0.f;
     if (sJ2 <= lim) {
-        y1[i] = 0.f;
-        y2[i] = 0.f;
         byield[i] = 0;
     } else if (lim > 0.f) {
-        y1[i] = 0.f;
-        y2[i] = (sJ2 - lim) / sJ2;
+        b = (sJ2 - lim) / sJ2;
     } else {
-        y1[i] = lim < -kEpsilon ? lim / (B * sD1) : 1.0f;
-        y2[i] = 1.0f;
+        a = lim < -kEpsilon ? lim / (B * sD1) : 1.0f;
+        b = 1.0f;
     }
+    y1[i] = a;
+    y2[i] = b;
     i1[i] = I1;
+    y4[i] = make_float4(a, b, I1, 0.f);  // gathered together by k_pl_yield
 }
 
 // v.norm() > EPSILON ? v.normalize() : 0 (normalize gives 0 below FLT_EPSILON).
@@ -362,33 +400,41 @@ __device__ inline void unit_or_zero3(float v[3])
 
 // PM_ApplyYielding (ElastoplasticityModule.cu:165-226).
 __global__ void __launch_bounds__(kPlBlock)
-    k_pl_yield(RestView R, const float* __restrict__ x, const float* __restrict__ y1, const float* __restrict__ y2,
-               const float* __restrict__ i1)
+    k_pl_yield(RestView R, const float4* __restrict__ x, const float4* __restrict__ y4)
 {
     const PlLane L = pl_lane(R.n);
     const int i = L.i;
     const long long a0 = pd_at(R.index, R.cap, i, 0);
     const float ri[3] = {R.rpos[3 * a0], R.rpos[3 * a0 + 1], R.rpos[3 * a0 + 2]};
     const int m = pd_size(R.index, R.cap, R.total, R.n, i);
+    const float4 xi = __ldg(x + i), yi = __ldg(y4 + i);
     __syncwarp();  // every lane has read slot 0 before lane 0 of the group rewrites it
     if (!L.valid) return;
-    for (int e = L.sub; e < m; e += kPlG) {
-        const long long at = pd_at(R.index, R.cap, i, e);
-        const int j = R.ridx[at];
-        float* rj = R.rpos + 3 * at;
-        const float s = i1[i] + i1[j];
-        const float ya = (y1[i] + y1[j]) / 2, yb = (y2[i] + y2[j]) / 2;
-        float p[3], q[3], nq[3], iso[3], dq[3];
-        for (int a = 0; a < 3; ++a) {
-            p[a] = x[3 * j + a] - x[3 * i + a];
-            q[a] = rj[a] - ri[a];
-            nq[a] = q[a] * s / 2;
-            iso[a] = nq[a] - q[a];
-            dq[a] = q[a];
+    for (int e0 = L.sub; e0 < m; e0 += kPlG * 2) {
+        float4 xj[2], yj[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int j = e0 + u * kPlG < m ? R.ridx[a0 + e0 + u * kPlG] : i;
+            xj[u] = __ldg(x + j);
+            yj[u] = __ldg(y4 + j);
         }
-        unit_or_zero3(dq);
-        const float pl = len3(p[0], p[1], p[2]);
-        for (int a = 0; a < 3; ++a) rj[a] = (rj[a] + ya * iso[a]) + yb * (pl * dq[a] - nq[a]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (e0 + u * kPlG >= m) break;
+            float* rj = R.rpos + 3 * (a0 + e0 + u * kPlG);
+            const float s = yi.z + yj[u].z;
+            const float ya = (yi.x + yj[u].x) / 2, yb = (yi.y + yj[u].y) / 2;
+            float q[3], nq[3], iso[3], dq[3];
+            for (int a = 0; a < 3; ++a) {
+                q[a] = rj[a] - ri[a];
+                nq[a] = q[a] * s / 2;
+                iso[a] = nq[a] - q[a];
+                dq[a] = q[a];
+            }
+            unit_or_zero3(dq);
+            const float pl = len3(xj[u].x - xi.x, xj[u].y - xi.y, xj[u].z - xi.z);
+            for (int a = 0; a < 3; ++a) rj[a] = (rj[a] + ya * iso[a]) + yb * (pl * dq[a] - nq[a]);
+        }
     }
 }
 
@@ -493,7 +539,7 @@ __global__ void __launch_bounds__(128)
 
 // FractureModule's PM_ComputeInvariants (FractureModule.cu:15-105).
 __global__ void __launch_bounds__(kPlBlock)
-    k_pl_fracture(RestView R, const float* __restrict__ x, float* __restrict__ bulk, float h, float A, float B,
+    k_pl_fracture(RestView R, const float4* __restrict__ x, float* __restrict__ bulk, float h, float A, float B,
                   float mu, float lambda)
 {
     const PlLane L = pl_lane(R.n);
@@ -523,11 +569,15 @@ int pl_rotate(pk_ctx* c, const float* x, float h, cudaStream_t st)
 {
     if (c->pd_n <= 0) return 0;
     const RestView R = rest_view(c);
+    int l = 0;
+    const float4* x4 = pd_pack(c, x, true, l, st);
+    if (!x4) return -1;
+    const BondView V{c->pd_bond, x4};
     const unsigned g = blocks((long long)c->pd_n * kPlG, kPlBlock);
-    k_pl_rot_sums<<<g, kPlBlock, 0, st>>>(R, x, h, c->pl_mk);
+    k_pl_rot_sums<<<g, kPlBlock, 0, st>>>(R, V, h, c->pl_mk);
     k_pl_rot_solve<<<blocks(c->pd_n, 128), 128, 0, st>>>(c->pd_n, h, c->pl_mk);
     k_pl_rot_apply<<<g, kPlBlock, 0, st>>>(R, c->pl_mk);
-    return 3;
+    return l + 3;
 }
 
 int pl_yield(pk_ctx* c, const float* x, const pk_plastic_params* p, cudaStream_t st)
@@ -535,20 +585,27 @@ int pl_yield(pk_ctx* c, const float* x, const pk_plastic_params* p, cudaStream_t
     const int n = c->pd_n;
     if (n <= 0) return 0;
     const RestView R = rest_view(c);
+    int l = 0;
+    const float4* x4 = pd_pack(c, x, false, l, st);
+    if (!x4) return -1;
     const unsigned g = blocks((long long)n * kPlG, kPlBlock);
-    k_pl_invariants<<<g, kPlBlock, 0, st>>>(R, x, c->pd_bulk, p->horizon, p->A, p->B, p->mu, p->lambda, c->pl_y1,
-                                            c->pl_y2, c->pl_i1, c->pl_yield);
-    k_pl_yield<<<g, kPlBlock, 0, st>>>(R, x, c->pl_y1, c->pl_y2, c->pl_i1);
-    return 2;
+    float4* const y4 = reinterpret_cast<float4*>(c->pl_mk);  // the rotation's scratch
+    k_pl_invariants<<<g, kPlBlock, 0, st>>>(R, x4, c->pd_bulk, p->horizon, p->A, p->B, p->mu, p->lambda, c->pl_y1,
+                                            c->pl_y2, c->pl_i1, c->pl_yield, y4);
+    k_pl_yield<<<g, kPlBlock, 0, st>>>(R, x4, y4);
+    return l + 2;
 }
 
 int pl_fracture(pk_ctx* c, const float* x, const pk_plastic_params* p, cudaStream_t st)
 {
     if (c->pd_n <= 0) return 0;
-    k_pl_fracture<<<blocks((long long)c->pd_n * kPlG, kPlBlock), kPlBlock, 0, st>>>(rest_view(c), x, c->pd_bulk,
+    int l = 0;
+    const float4* x4 = pd_pack(c, x, false, l, st);
+    if (!x4) return -1;
+    k_pl_fracture<<<blocks((long long)c->pd_n * kPlG, kPlBlock), kPlBlock, 0, st>>>(rest_view(c), x4, c->pd_bulk,
                                                                                     p->horizon, p->A, p->B, p->mu,
                                                                                     p->lambda);
-    return 1;
+    return l + 1;
 }
 
 int pl_enable_all(pk_ctx* c, cudaStream_t st)
