@@ -414,7 +414,9 @@ __device__ __forceinline__ Q4<R> gather_slots(const PdBonds& B, const Q4<R>* __r
 // weight rides in its slot's fourth value, so W follows broken bonds and
 // changed stiffness without a pass of its own).  kLast writes the caller's x
 // (3 per particle) and, with v, v += (xn - xold)/dt (K_UpdateVelocity,
-// ElasticityModule.cu:295-306) instead of the next iterate.
+// ElasticityModule.cu:295-306) instead of the next iterate.  Bound by the
+// scattered 16-byte slots; four in flight per lane: 154 us per launch at 524,288
+// particles with 80 bonds, one ahead 184.
 template <class R, bool kLast>
 __global__ void __launch_bounds__(kPdBlock)
     k_pd_gather(PdBonds B, const Q4<R>* __restrict__ x, const Q4<R>* __restrict__ xold,
@@ -616,7 +618,9 @@ __global__ void __launch_bounds__(kPdBlock, 4)
 
 // g = dL/dx of the iterate.  Unless it is the step's first iterate, what the
 // previous iteration's reverse needs comes with it: a = g/(1 + W) and
-// xoldbar += a; the first iterate's g is kept for k_pd_adj_tail.
+// xoldbar += a; the first iterate's g is kept for k_pd_adj_tail.  Bound by the
+// scattered 32-byte slots; at 65,536 particles with 80 bonds 46 us per launch,
+// 49 and 3.3 as two kernels.
 template <class R>
 __global__ void __launch_bounds__(kPdBlock)
     k_pd_adjC_gather(PdBonds B, const Q4<R>* __restrict__ gown, const Q4<R>* __restrict__ slot,
